@@ -7,7 +7,7 @@
 // :93-104), rank-1 update (Rank1Update :38-50), stop at the first exactly-zero pivot
 // (:127-137). The B200 kernels are:
 //   n <= 32 : getrf_small_kernel, one warp segment per matrix, rows in registers;
-//   32 < n <= 128 : getrf_reg_kernel (getrf_reg.cu), matrix in registers across the CTA;
+//   32 < n <= 128 : getrf_mid_kernel (getrf_mid.cu), blocked in shared memory, one CTA per matrix;
 //   128 < n <= 1024 : the blocked LU on a by-rows copy made in place (getrf_blocked_tc.cu:
 //                     panel kernels and a tiled trailing update), given 4 bytes of handle
 //                     workspace per matrix; without them getrf_large_kernel (getrf_large.cu,
@@ -220,11 +220,8 @@ aclblasStatus_t opsblas::getrf_batched_impl(aclblasHandle_t handle, int n, float
             default:
                 break;
         }
-    } else if (getrf_reg_supported(n)) {
-        int rows, warps;
-        reg_default_shape(n, rows, warps);
-        return launch_status(kApi, getrf_reg_launch(st, Aarray, n, lda, PivotArray, infoArray, batchSize, rows,
-                                                    warps));
+    } else if (getrf_mid_supported(n)) {
+        return launch_status(kApi, getrf_mid_launch(st, Aarray, n, lda, PivotArray, infoArray, batchSize));
     } else if (getrf_rows_supported(n, batchSize) && stat != nullptr) {
         return launch_status(kApi, getrf_rows_launch(st, Aarray, n, lda, PivotArray, infoArray, stat, batchSize));
     } else if (getrf_large_supported(n)) {

@@ -9,13 +9,12 @@
 // (32 < n <= 128) from a tuning table written by autotune_grouped.py (or from the caller),
 // orders the work largest first, and uploads the task lists to the device. Each execution is
 // then one launch of grouped_lu_kernel on the handle's stream (plus the regular batched kernels
-// for groups with n > 128): a grid of one wave of 256-thread CTAs that take tasks from two
-// device counters --
-//   phase 1, CTA tasks (n > 32): the CTA (8 warps) or each 4-warp / 2-warp team factors one matrix
-//     held in registers (reg_getrf_core), stores LU, pivots and info, and solves the
-//     right-hand sides from a copy of the factors in shared memory (med_solve_core);
-//   phase 2, warp tasks (n <= 32): each warp takes 32/lanes matrices, factors them in
-//     registers (small_getrf_core) and solves from the registers (small_solve_core).
+// for groups with n > 128): one CTA of twelve warps an SM, whose teams take tasks from a device
+// counter per class of orders, largest class first --
+//   n > 32: teams of 4, 2 or 1 warps factor one matrix in their share of the CTA's shared memory
+//     (lu_mid.cuh), solve the right-hand sides from there (mid_solve) and store LU, pivots and info;
+//   n <= 32: each warp takes 32/lanes matrices, factors them in registers (small_getrf_core) and
+//     solves from the registers (small_solve_core).
 // The last CTA to finish resets the counters, so consecutive executions on one stream need no
 // host work, and executions of one plan must not overlap in time.
 #include <cuda_runtime.h>
@@ -29,10 +28,11 @@
 
 #include "internal.h"
 #include "lu_core.cuh"
+#include "lu_mid.cuh"
 
 namespace opsblas {
 
-constexpr int kGrpThreads = 256;
+constexpr int kGrpThreads = 384;
 constexpr int kGrpWarps = kGrpThreads / 32;
 constexpr int kGrpMaxN = 128;  // larger orders use the batched kernels
 
@@ -41,9 +41,6 @@ struct GroupDev {
     long long piv_off;  // first pivot of the group's first instance
     int first;          // index of the group's first instance in the pointer arrays
     int lanes;          // n <= 32: lanes per matrix (SEG)
-    int warps;          // n > 32: warps per matrix (2, 4 or 8)
-    int rows;           // n > 32: rows per lane (2, 3 or 4; 32 * rows >= n)
-    int team_floats;    // n > 32: shared-memory floats between consecutive teams' staged factors
     int pad;
 };
 
@@ -55,90 +52,49 @@ struct GroupTask {
 };
 
 // ------------------------------------------------------------------------------ n > 32 --
-// One matrix per team of NW warps: registers hold the matrix (reg_getrf_core). With right-hand
-// sides, the factors are also staged in the team's shared memory (physical rows, odd column
-// stride) so that the team's warps solve their columns from there (med_solve_core) while the
-// factors go to global memory.
-template <int R, int NW>
-__device__ __forceinline__ void grouped_reg(const GroupDev& g, int li, float* const* Aarray, float* const* Barray,
-                                            int* piv, int* info, RegTeamSmem& S, float* sa, int warp, int lane,
-                                            int bar)
+// One matrix per team of W warps, factored in the team's shared memory (lu_mid.cuh); the right-hand
+// sides are solved from there, one per warp, while the factors go to global memory. bar: W barriers
+// of the panels, then the team's own.
+template <int NBLK, int W>
+__device__ __forceinline__ void grouped_mid(const GroupDev& g, int li, float* const* Aarray, float* const* Barray,
+                                            int* piv, int* info, void* region, int warp, int lane, int bar)
 {
-    constexpr int CW = RegShape<R, NW>::CW;
+    constexpr int R = MidSmem<NBLK, W>::R;
+    auto& M = *static_cast<MidSmem<NBLK, W>*>(region);
     const int n = g.n;
     const long long inst = (long long)g.first + li;
     float* A = Aarray[inst];
-    int* pm = piv + g.piv_off + (long long)li * n;
-    float a[R][CW];
-    int pos[R];
-    reg_load<R, NW>(a, A, g.lda, n, warp, lane);
+    mid_stage<NBLK, W>(M, A, g.lda, n, warp, lane);
+    if (warp == 0 && lane == 0) M.stop = n;
+    cp_async_wait_all();
+    team_sync<W * 32>(bar + W);
+    mid_getrf<NBLK, true, W, 0>(M, n, warp, lane, bar);
+    team_sync<W * 32>(bar + W);
+    for (int c = warp; c < g.nrhs; c += W) {
+        float* bc = Barray[inst] + (long long)c * g.ldb;
+        float y[R];
 #pragma unroll
-    for (int t = 0; t < R; t++) pos[t] = lane + 32 * t;
-    for (int i = warp * 32 + lane; i < n; i += NW * 32) pm[i] = 0;
-    team_sync<NW * 32>(bar);
-    const int inf = reg_getrf_core<R, NW, true>(a, pos, n, S, pm, warp, lane, bar);
-    const int ld = n | 1;
-    if (g.nrhs > 0) {
+        for (int t = 0; t < R; t++) y[t] = lane + 32 * t < n ? bc[M.rowof[lane + 32 * t]] : 0.0f;
+        __syncwarp();  // every lane has read its b before any lane writes x
+        mid_solve<NBLK, W>(M, n, lane, y);
 #pragma unroll
-        for (int s = 0; s < CW; s++) {
-            const int j = s * NW + warp;
-#pragma unroll
-            for (int t = 0; t < R; t++) {
-                const int p = lane + 32 * t;
-                if (p < n && j < n) sa[p + j * ld] = a[t][s];
-            }
-        }
-        if (warp == 0) {
-#pragma unroll
-            for (int t = 0; t < R; t++)
-                if (lane + 32 * t < n) S.lmap[pos[t]] = lane + 32 * t;
-        }
+        for (int t = 0; t < R; t++)
+            if (lane + 32 * t < n) bc[lane + 32 * t] = y[t];
     }
-    reg_store<R, NW>(a, pos, A, g.lda, n, warp, lane);
-    if (g.nrhs > 0) {
-        team_sync<NW * 32>(bar);  // staged factors and row map visible to the team
-        float* Bm = Barray[inst];
-        for (int c = warp; c < g.nrhs; c += NW) {
-            float* bc = Bm + (long long)c * g.ldb;
-            float y[kMedRows];
-#pragma unroll
-            for (int t = 0; t < kMedRows; t++) {
-                const int i = lane + 32 * t;
-                y[t] = i < n ? bc[S.lmap[i]] : 0.0f;
-            }
-            __syncwarp();  // every lane has read its b before any lane writes x
-            med_solve_core(sa, S.lmap, n, ld, lane, y);
-            __syncwarp();
-#pragma unroll
-            for (int t = 0; t < kMedRows; t++) {
-                const int i = lane + 32 * t;
-                if (i < n) bc[i] = y[t];
-            }
-        }
-    }
-    if (warp == 0 && lane == 0) info[inst] = inf;
+    mid_store<NBLK, W>(M, A, g.lda, n, piv + g.piv_off + (long long)li * n, warp, lane);
+    if (warp == 0 && lane == 0) info[inst] = M.stop < n ? M.stop + 1 : 0;
 }
 
-template <int NW>
-__device__ __forceinline__ void grouped_reg_dispatch(const GroupDev& g, int li, float* const* Aarray,
-                                                     float* const* Barray, int* piv, int* info, RegTeamSmem& S,
-                                                     float* sa, int warp, int lane, int bar)
+// Classes of orders and how the CTA's twelve warps and its shared memory are dealt out to each: as many
+// matrices at a time as the memory holds, 4 warps each above 96 rows, 2 above 64, 1 below.
+constexpr int kGrpClasses = 5;  // 97..128, 81..96, 65..80, 33..64, 1..32
+__host__ __device__ constexpr int grp_class(int n) { return n > 96 ? 0 : n > 80 ? 1 : n > 64 ? 2 : n > 32 ? 3 : 4; }
+__host__ __device__ constexpr int grp_team_warps(int c) { return c == 0 ? 4 : c < 3 ? 2 : 1; }
+__host__ __device__ constexpr int grp_teams(int c) { return c == 0 ? 3 : c < 3 ? 5 : c == 3 ? 11 : 12; }
+__host__ __device__ constexpr size_t grp_region(int c)
 {
-    if (NW == 2) {
-        grouped_reg<2, 2>(g, li, Aarray, Barray, piv, info, S, sa, warp, lane, bar);
-    } else if (NW == 4) {
-        if (g.rows == 2)
-            grouped_reg<2, 4>(g, li, Aarray, Barray, piv, info, S, sa, warp, lane, bar);
-        else
-            grouped_reg<3, 4>(g, li, Aarray, Barray, piv, info, S, sa, warp, lane, bar);
-    } else {
-        if (g.rows == 2)
-            grouped_reg<2, 8>(g, li, Aarray, Barray, piv, info, S, sa, warp, lane, bar);
-        else if (g.rows == 3)
-            grouped_reg<3, 8>(g, li, Aarray, Barray, piv, info, S, sa, warp, lane, bar);
-        else
-            grouped_reg<4, 8>(g, li, Aarray, Barray, piv, info, S, sa, warp, lane, bar);
-    }
+    return c == 0 ? sizeof(MidSmem<8, 4>) : c == 1 ? sizeof(MidSmem<6, 2>) : c == 2 ? sizeof(MidSmem<5, 2>)
+           : c == 3 ? sizeof(MidSmem<4, 1>) : 3 * 32 * sizeof(float);  // small: two row buffers, owners
 }
 
 // ----------------------------------------------------------------------------- n <= 32 --
@@ -196,73 +152,95 @@ __device__ __forceinline__ void grouped_small_dispatch(const GroupDev& g, const 
         grouped_small<N, 32>(g, task, Aarray, Barray, piv, info, rowbuf, owner, lane);
 }
 
-__global__ void __launch_bounds__(kGrpThreads, 2)
-grouped_lu_kernel(const GroupDev* groups, const GroupTask* __restrict__ cta_tasks, int n_cta,
-                  const GroupTask* __restrict__ warp_tasks, int n_warp, int* __restrict__ counters,
-                  float* const* Aarray, float* const* Barray, int* piv, int* info)
+// Tasks of one class, taken by the CTA's teams from the class's counter.
+template <int C>
+__device__ __forceinline__ void grouped_class(const GroupDev* groups, const GroupTask* __restrict__ tasks, int count,
+                                              int* counter, float* const* Aarray, float* const* Barray, int* piv,
+                                              int* info, unsigned char* dyn, int* s_task, int wid, int lane)
 {
-    extern __shared__ __align__(16) float dyn[];  // per team: staged factors for the solve
-    __shared__ RegTeamSmem team[4];
-    __shared__ int s_task;
-    __shared__ __align__(16) float rowbuf[kGrpWarps][2][32];
-    __shared__ int owner[kGrpWarps][32];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-
-    // phase 1: one matrix per CTA (or per 4-warp team), largest first
+    constexpr int W = grp_team_warps(C);
+    const int team = wid / W, warp = wid % W;
+    if (team >= grp_teams(C)) return;
+    const int bar = 1 + team * (W + 1);
+    unsigned char* region = dyn + (size_t)team * grp_region(C);
     for (;;) {
-        if (tid == 0) s_task = atomicAdd(&counters[0], 1);
-        __syncthreads();
-        const int t = s_task;
-        __syncthreads();
-        if (t >= n_cta) break;
-        const GroupTask task = cta_tasks[t];
-        const GroupDev& g = groups[task.group];  // fields read when needed: fewer live registers
-        if (g.warps == 2) {  // four 2-warp teams, one matrix each
-            const int tm = warp >> 1;
-            if (tm < task.count)
-                grouped_reg_dispatch<2>(g, task.first + tm, Aarray, Barray, piv, info, team[tm],
-                                        dyn + (size_t)tm * g.team_floats, warp & 1, lane, 1 + tm);
-        } else if (g.warps == 4) {
-            const int tm = warp >> 2;
-            if (tm < task.count)
-                grouped_reg_dispatch<4>(g, task.first + tm, Aarray, Barray, piv, info, team[tm],
-                                        dyn + (size_t)tm * g.team_floats, warp & 3, lane,
-                                        1 + tm);
+        team_sync<W * 32>(bar + W);  // the previous task's shared memory and task number are done with
+        int t;
+        if (W == 1) {
+            t = lane == 0 ? atomicAdd(counter, 1) : 0;
+            t = __shfl_sync(0xffffffffu, t, 0);
         } else {
-            grouped_reg_dispatch<8>(g, task.first, Aarray, Barray, piv, info, team[0], dyn, warp, lane, -1);
+            if (warp == 0 && lane == 0) s_task[team] = atomicAdd(counter, 1);
+            team_sync<W * 32>(bar + W);
+            t = s_task[team];
         }
-    }
-
-    // phase 2: warp tasks, each warp on its own
-    for (;;) {
-        __syncwarp();  // the previous task's shared-memory reads are done before rowbuf is reused
-        int t = 0;
-        if (lane == 0) t = atomicAdd(&counters[1], 1);
-        t = __shfl_sync(0xffffffffu, t, 0);
-        if (t >= n_warp) break;
-        const GroupTask task = warp_tasks[t];
-        const GroupDev g = groups[task.group];
-        switch (g.n) {
+        if (t >= count) break;
+        const GroupTask task = tasks[t];
+        const GroupDev& g = groups[task.group];  // fields read when needed: fewer live registers
+        if constexpr (C == 0) {
+            if (g.n > 112)
+                grouped_mid<8, W>(g, task.first, Aarray, Barray, piv, info, region, warp, lane, bar);
+            else
+                grouped_mid<7, W>(g, task.first, Aarray, Barray, piv, info, region, warp, lane, bar);
+        } else if constexpr (C == 1) {
+            grouped_mid<6, W>(g, task.first, Aarray, Barray, piv, info, region, warp, lane, bar);
+        } else if constexpr (C == 2) {
+            grouped_mid<5, W>(g, task.first, Aarray, Barray, piv, info, region, warp, lane, bar);
+        } else if constexpr (C == 3) {
+            if (g.n > 48)
+                grouped_mid<4, W>(g, task.first, Aarray, Barray, piv, info, region, warp, lane, bar);
+            else
+                grouped_mid<3, W>(g, task.first, Aarray, Barray, piv, info, region, warp, lane, bar);
+        } else {
+            float* rowbuf = reinterpret_cast<float*>(region);
+            int* owner = reinterpret_cast<int*>(rowbuf + 64);
+            switch (g.n) {
 #define OPSBLAS_GROUPED_CASE(NN)                                                                                    \
     case NN:                                                                                                        \
-        grouped_small_dispatch<NN>(g, task, Aarray, Barray, piv, info, &rowbuf[warp][0][0], owner[warp], lane);     \
+        grouped_small_dispatch<NN>(g, task, Aarray, Barray, piv, info, rowbuf, owner, lane);                        \
         break;
-            OPSBLAS_FOR_N_1_32(OPSBLAS_GROUPED_CASE)
+                OPSBLAS_FOR_N_1_32(OPSBLAS_GROUPED_CASE)
 #undef OPSBLAS_GROUPED_CASE
-            default:
-                break;
+                default:
+                    break;
+            }
         }
     }
+}
+
+// One CTA an SM. The classes follow each other, largest orders first; within a class every team works
+// on its own. tasks: the classes' lists one after the other, class c at [first[c], first[c + 1]).
+// counters: one a class, then the CTAs that are done.
+struct GroupLists {
+    int first[kGrpClasses + 1];
+};
+
+__global__ void __launch_bounds__(kGrpThreads, 1)
+grouped_lu_kernel(const GroupDev* groups, const GroupTask* __restrict__ tasks, const GroupLists lists,
+                  int* __restrict__ counters, float* const* Aarray, float* const* Barray, int* piv, int* info)
+{
+    extern __shared__ __align__(16) unsigned char dyn[];
+    __shared__ int s_task[kGrpWarps];
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#define OPSBLAS_GROUPED_CLASS(C)                                                                                    \
+    if (lists.first[C + 1] > lists.first[C]) {                                                                      \
+        grouped_class<C>(groups, tasks + lists.first[C], lists.first[C + 1] - lists.first[C], counters + C, Aarray, \
+                         Barray, piv, info, dyn, s_task, wid, lane);                                                \
+        __syncthreads();                                                                                            \
+    }
+    OPSBLAS_GROUPED_CLASS(0)
+    OPSBLAS_GROUPED_CLASS(1)
+    OPSBLAS_GROUPED_CLASS(2)
+    OPSBLAS_GROUPED_CLASS(3)
+    OPSBLAS_GROUPED_CLASS(4)
+#undef OPSBLAS_GROUPED_CLASS
 
     // the last CTA out resets the counters for the next execution
-    __syncthreads();
-    if (tid == 0) {
+    if (threadIdx.x == 0) {
         __threadfence();
-        const int f = atomicAdd(&counters[2], 1);
+        const int f = atomicAdd(&counters[kGrpClasses], 1);
         if (f == (int)gridDim.x - 1) {
-            atomicExch(&counters[0], 0);
-            atomicExch(&counters[1], 0);
-            atomicExch(&counters[2], 0);
+            for (int c = 0; c <= kGrpClasses; c++) atomicExch(&counters[c], 0);
         }
     }
 }
@@ -272,7 +250,22 @@ struct TuneRow {
     int lo, hi, lanes, warps, rows;
 };
 
-// Built-in choices, used when no tuning table is found: natural lanes; 8 warps, ceil(n/32) rows.
+// Choices for n > 32 (rows per lane, warps per matrix) that a configuration or the table may name:
+// checked and reported as ever; the kernel deals out its warps by the order alone (grp_class).
+static bool reg_shape_valid(int n, int rows, int warps)
+{
+    if (n <= 32 || n > 32 * rows) return false;
+    return (rows == 2 && (warps == 2 || warps == 4 || warps == 8)) || (rows == 3 && (warps == 4 || warps == 8)) ||
+           (rows == 4 && warps == 8);
+}
+
+static void reg_default_shape(int n, int& rows, int& warps)
+{
+    rows = (n + 31) / 32;
+    warps = rows == 2 ? 2 : (rows == 3 ? 4 : 8);
+}
+
+// Built-in choices, used when no tuning table is found.
 static void default_config(int n, int cfg[3])
 {
     if (n <= 32) {
@@ -347,10 +340,9 @@ struct _aclblas_grouped_plan {
     int total = 0;
     void* dmem = nullptr;
     opsblas::GroupDev* d_groups = nullptr;
-    opsblas::GroupTask* d_cta = nullptr;
-    opsblas::GroupTask* d_warp = nullptr;
+    opsblas::GroupTask* d_tasks = nullptr;
     int* d_counters = nullptr;
-    int n_cta = 0, n_warp = 0;
+    opsblas::GroupLists lists = {};
     int grid = 0;
     size_t smem = 0;      // dynamic shared memory per CTA
     bool has_persistent = false;
@@ -429,58 +421,43 @@ extern "C" aclblasStatus_t aclblasSgetrfGetrsGroupedPlanCreate(aclblasHandle_t h
     std::vector<int> order(groupCount);
     for (int g = 0; g < groupCount; g++) order[g] = g;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return p->groups[a].n > p->groups[b].n; });
-    std::vector<GroupTask> cta, warp;
+    std::vector<GroupTask> tasks;
     size_t smem = 0;
-    std::vector<int> team_stride(std::max(groupCount, 1), 0);
+    int cls = 0;
     for (int g : order) {
         const GroupHost& h = p->groups[g];
         if (h.n == 0 || h.size == 0 || h.n > kGrpMaxN) continue;
-        if (h.n > 32) {
-            const int per = kGrpWarps / h.cfg[1];  // matrices per CTA task (teams)
-            for (int i = 0; i < h.size; i += per) cta.push_back({g, i, std::min(per, h.size - i), 0});
-            if (h.nrhs > 0) {
-                // staged factors, 16-byte rounded; team t's region starts at t * f, the teams of a
-                // CTA stage side by side
-                const size_t f = ((size_t)(h.n | 1) * h.n + 3) & ~(size_t)3;
-                team_stride[g] = (int)f;
-                smem = std::max(smem, (size_t)per * f * 4);
-            }
-        } else {
-            const int per = 32 / h.cfg[0];
-            for (int i = 0; i < h.size; i += per) warp.push_back({g, i, std::min(per, h.size - i), 0});
-        }
+        const int c = grp_class(h.n);
+        while (cls < c) p->lists.first[++cls] = (int)tasks.size();
+        smem = std::max(smem, grp_teams(c) * grp_region(c));
+        const int per = h.n > 32 ? 1 : 32 / h.cfg[0];  // matrices a task
+        for (int i = 0; i < h.size; i += per) tasks.push_back({g, i, std::min(per, h.size - i), 0});
     }
-    p->n_cta = (int)cta.size();
-    p->n_warp = (int)warp.size();
-    p->has_persistent = p->n_cta + p->n_warp > 0;
+    while (cls < kGrpClasses) p->lists.first[++cls] = (int)tasks.size();
+    p->has_persistent = !tasks.empty();
     p->smem = smem;
 
     std::vector<GroupDev> gd(std::max(groupCount, 1));
     for (int g = 0; g < groupCount; g++) {
         const GroupHost& h = p->groups[g];
-        gd[g] = {h.n, h.nrhs, h.lda, h.ldb, h.piv_off, h.first, h.cfg[0], h.cfg[1], h.cfg[2], team_stride[g], 0};
+        gd[g] = {h.n, h.nrhs, h.lda, h.ldb, h.piv_off, h.first, h.cfg[0], 0};
     }
     if (p->has_persistent) {
         const size_t bg = gd.size() * sizeof(GroupDev);
-        const size_t bc = std::max<size_t>(cta.size(), 1) * sizeof(GroupTask);
-        const size_t bw = std::max<size_t>(warp.size(), 1) * sizeof(GroupTask);
-        cudaError_t err = cudaMalloc(&p->dmem, bg + bc + bw + 256);
+        const size_t bt = tasks.size() * sizeof(GroupTask);
+        cudaError_t err = cudaMalloc(&p->dmem, bg + bt + 256);
         if (err != cudaSuccess) {
-            log_error(kApi, "cannot allocate %zu bytes for the plan", bg + bc + bw + 256);
+            log_error(kApi, "cannot allocate %zu bytes for the plan", bg + bt + 256);
             delete p;
             return ACLBLAS_STATUS_ALLOC_FAILED;
         }
         char* d = static_cast<char*>(p->dmem);
         p->d_counters = reinterpret_cast<int*>(d);
         p->d_groups = reinterpret_cast<GroupDev*>(d + 256);
-        p->d_cta = reinterpret_cast<GroupTask*>(d + 256 + bg);
-        p->d_warp = reinterpret_cast<GroupTask*>(d + 256 + bg + bc);
+        p->d_tasks = reinterpret_cast<GroupTask*>(d + 256 + bg);
         err = cudaMemset(p->d_counters, 0, 256);
         if (err == cudaSuccess) err = cudaMemcpy(p->d_groups, gd.data(), bg, cudaMemcpyHostToDevice);
-        if (err == cudaSuccess && !cta.empty())
-            err = cudaMemcpy(p->d_cta, cta.data(), cta.size() * sizeof(GroupTask), cudaMemcpyHostToDevice);
-        if (err == cudaSuccess && !warp.empty())
-            err = cudaMemcpy(p->d_warp, warp.data(), warp.size() * sizeof(GroupTask), cudaMemcpyHostToDevice);
+        if (err == cudaSuccess) err = cudaMemcpy(p->d_tasks, tasks.data(), bt, cudaMemcpyHostToDevice);
         if (err == cudaSuccess)
             err = ensure_smem_limit(grouped_lu_kernel, (int)std::max<size_t>(p->smem, 1));
         int per_sm = 0;
@@ -492,8 +469,7 @@ extern "C" aclblasStatus_t aclblasSgetrfGetrsGroupedPlanCreate(aclblasHandle_t h
             delete p;
             return err != cudaSuccess ? launch_status(kApi, err) : ACLBLAS_STATUS_NOT_SUPPORTED;
         }
-        const long long want = (long long)p->n_cta + (p->n_warp + kGrpWarps - 1) / kGrpWarps;
-        p->grid = (int)std::max(1LL, std::min<long long>(want, (long long)per_sm * sm_count()));
+        p->grid = (int)std::min<long long>((long long)tasks.size(), sm_count());
     }
     *plan = p;
     return ACLBLAS_STATUS_SUCCESS;
@@ -542,8 +518,7 @@ extern "C" aclblasStatus_t aclblasSgetrfGetrsGroupedBatched(aclblasHandle_t hand
     cudaStream_t st = handle->stream;
     if (plan->has_persistent) {
         grouped_lu_kernel<<<(unsigned)plan->grid, kGrpThreads, plan->smem, st>>>(
-            plan->d_groups, plan->d_cta, plan->n_cta, plan->d_warp, plan->n_warp, plan->d_counters, Aarray, Barray,
-            PivotArray, infoArray);
+            plan->d_groups, plan->d_tasks, plan->lists, plan->d_counters, Aarray, Barray, PivotArray, infoArray);
         cudaError_t err = cudaGetLastError();
         if (err != cudaSuccess) return launch_status(kApi, err);
     }

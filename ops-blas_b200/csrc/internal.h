@@ -155,11 +155,8 @@ cudaError_t getrf_tmem_launch(cudaStream_t st, const float* const* Aarray, int l
 bool getrf_large_supported(int n);
 cudaError_t getrf_large_launch(cudaStream_t st, float* const* Aarray, int n, int lda, int* piv, int* info, int batch);
 
-// getrf_reg.cu: 32 < n <= 128, matrix in registers; shape = rows per lane x warps per matrix.
-bool getrf_reg_supported(int n);
-bool reg_shape_valid(int n, int rows, int warps);
-void reg_default_shape(int n, int& rows, int& warps);
-cudaError_t getrf_reg_launch(cudaStream_t st, float* const* Aarray, int n, int lda, int* piv, int* info, int batch,
-                             int rows, int warps);
+// getrf_mid.cu: 32 < n <= 128, blocked LU of a matrix in shared memory.
+bool getrf_mid_supported(int n);
+cudaError_t getrf_mid_launch(cudaStream_t st, float* const* Aarray, int n, int lda, int* piv, int* info, int batch);
 
 }  // namespace opsblas

@@ -1,4 +1,4 @@
-// LU building blocks shared by the batched kernels (getrf.cu, getrf_reg.cu) and the grouped
+// LU building blocks shared by the batched kernels (getrf.cu) and the grouped
 // persistent kernel (grouped.cu). Each block restates the reference's unblocked right-looking
 // LU (sgetrf_batched_kernel.cpp:106-150): first-maximum pivot, whole-row interchange,
 // multipliers by true division, one fmaf per update in column order, stop at the first
@@ -173,253 +173,6 @@ __device__ __forceinline__ void team_sync(int bar)
         __syncthreads();
     else
         asm volatile("bar.sync %0, %1;\n" ::"r"(bar), "n"(NT) : "memory");
-}
-
-// =============================================================================================
-// Register LU for 32 < n <= 128, run by a team of NW warps. The matrix lives in registers:
-// lane l of every warp holds rows p = l + 32 t (t < R, R = ceil(n / 32)), and warp w holds the
-// columns j = s * NW + w (slot s < CW = 32 R / NW), so every warp sees every row and the columns
-// are dealt out cyclically (all warps stay busy until the last columns). Pivoting is implicit as
-// in small_getrf_core: `pos` (replicated in every warp) is the row's index in the reference's
-// in-place matrix; rows never move. Per column k (owner warp k % NW, slot k / NW):
-//   A. the owner warp finds the first-maximum pivot (lane-local over t, then redux.sync),
-//      forms l = a / pivot for the rows that end below the pivot (true division) and publishes
-//      the pivot position, the pivot value and the multipliers in shared memory;
-//   B. one team barrier; every warp applies the interchange to `pos`, broadcasts the pivot row's
-//      entries of its own columns through shared memory, and updates a(i, j) -= l_i * u_j for
-//      its columns j > k and rows below the pivot -- one fmaf per element, column order.
-// On an exactly-zero pivot every warp stops (the reference's early exit).
-// =============================================================================================
-template <int R, int NW>
-struct RegShape {
-    static constexpr int NMAX = 32 * R;
-    static constexpr int CW = NMAX / NW;  // column slots per warp
-    static_assert(NMAX % NW == 0 && CW % 4 == 0, "columns must deal out evenly, in float4 chunks");
-};
-
-// Shared state of one team.
-struct __align__(16) RegTeamSmem {
-    float l[2][128];               // multipliers of the current column by physical row (double buffered)
-    float u[128];                  // the pivot row's entries; warp w's columns at u[w * CW]
-    int lmap[128];                 // after factoring: logical row -> physical row
-    int ppos[2];
-    float pv[2];
-};
-
-// Loads matrix A (n x n, leading dimension lda) into the team's registers.
-template <int R, int NW>
-__device__ __forceinline__ void reg_load(float (&a)[R][RegShape<R, NW>::CW], const float* A, int lda, int n,
-                                         int warp, int lane)
-{
-    constexpr int CW = RegShape<R, NW>::CW;
-#pragma unroll
-    for (int s = 0; s < CW; s++) {
-        const int j = s * NW + warp;
-#pragma unroll
-        for (int t = 0; t < R; t++) {
-            const int p = lane + 32 * t;
-            a[t][s] = (p < n && j < n) ? A[p + (long long)j * lda] : 0.0f;
-        }
-    }
-}
-
-// Stores the factors: row p goes to its final position pos.
-template <int R, int NW>
-__device__ __forceinline__ void reg_store(const float (&a)[R][RegShape<R, NW>::CW], const int (&pos)[R], float* A,
-                                          int lda, int n, int warp, int lane)
-{
-    constexpr int CW = RegShape<R, NW>::CW;
-#pragma unroll
-    for (int s = 0; s < CW; s++) {
-        const int j = s * NW + warp;
-#pragma unroll
-        for (int t = 0; t < R; t++) {
-            const int p = lane + 32 * t;
-            if (p < n && j < n) A[pos[t] + (long long)j * lda] = a[t][s];
-        }
-    }
-}
-
-// Factors the team's matrix. pos must start as the physical row (lane + 32 t); pm (when
-// pivoting) must be zero for the whole team before the call (a team barrier after zeroing).
-// Returns info.
-template <int R, int NW, bool PIVOT>
-__device__ __forceinline__ int reg_getrf_core(float (&a)[R][RegShape<R, NW>::CW], int (&pos)[R], int n,
-                                              RegTeamSmem& S, int* pm, int warp, int lane, int bar)
-{
-    constexpr int CW = RegShape<R, NW>::CW;
-    int info = 0;
-    bool stop = false;
-#pragma unroll
-    for (int c = 0; c < CW; c++) {
-        if (stop) break;
-        for (int w = 0; w < NW; w++) {
-            const int k = c * NW + w;
-            if (k >= n) {
-                stop = true;
-                break;
-            }
-            const int buf = k & 1;
-            if (warp == w) {
-                // ---- A: pivot, multipliers (owner warp) ----
-                int ppos = k;
-                if (PIVOT) {
-                    unsigned bkey = 0, bpos = 0xffffffffu;
-#pragma unroll
-                    for (int t = 0; t < R; t++) {
-                        const bool elig = pos[t] < n && pos[t] >= k;
-                        const float v = fabsf(a[t][c]);
-                        const unsigned key = (elig && v > 0.0f) ? __float_as_uint(v) : 0u;
-                        if (elig && (key > bkey || (key == bkey && (unsigned)pos[t] < bpos))) {
-                            bkey = key;
-                            bpos = (unsigned)pos[t];
-                        }
-                    }
-                    ppos = (int)seg_argmax<32>(bkey, bpos, 0);
-                }
-                float cand = 0.0f;
-                bool own = false;
-#pragma unroll
-                for (int t = 0; t < R; t++) {
-                    if (pos[t] == ppos) {
-                        cand = a[t][c];
-                        own = true;
-                    }
-                }
-                const unsigned bal = __ballot_sync(0xffffffffu, own);
-                const float pv = __shfl_sync(0xffffffffu, cand, __ffs(bal) - 1);
-                if (pv != 0.0f) {
-#pragma unroll
-                    for (int t = 0; t < R; t++) {
-                        const int np = pos[t] == ppos ? k : (pos[t] == k ? ppos : pos[t]);
-                        if (np > k && np < n) {
-                            const float l = a[t][c] / pv;
-                            a[t][c] = l;
-                            if (NW > 1) S.l[buf][lane + 32 * t] = l;
-                        }
-                    }
-                }
-                if (lane == 0) {
-                    S.ppos[buf] = ppos;
-                    S.pv[buf] = pv;
-                    if (PIVOT) pm[k] = ppos + 1;
-                }
-            }
-            team_sync<NW * 32>(bar);
-            // ---- B: interchange, pivot-row broadcast, update (every warp) ----
-            const int ppos = S.ppos[buf];
-            if (S.pv[buf] == 0.0f) {
-                info = k + 1;
-                stop = true;
-                break;
-            }
-#pragma unroll
-            for (int t = 0; t < R; t++) pos[t] = pos[t] == ppos ? k : (pos[t] == k ? ppos : pos[t]);
-            float l[R];
-            bool below[R];
-#pragma unroll
-            for (int t = 0; t < R; t++) {
-                below[t] = pos[t] > k && pos[t] < n;
-                l[t] = below[t] ? (NW == 1 ? a[t][c] : S.l[buf][lane + 32 * t]) : 0.0f;
-            }
-            // the lane holding logical row k publishes its slots (from chunk c/4 on) as float4s
-            float4* ub4 = reinterpret_cast<float4*>(S.u + warp * CW);
-#pragma unroll
-            for (int t = 0; t < R; t++) {
-                if (pos[t] == k) {
-#pragma unroll
-                    for (int q = c / 4; q < CW / 4; q++)
-                        ub4[q] = make_float4(a[t][4 * q], a[t][4 * q + 1], a[t][4 * q + 2], a[t][4 * q + 3]);
-                }
-            }
-            __syncwarp();
-            // update, one float4 chunk of the pivot row at a time (slot c only for warps after the
-            // owner; slots > c always), two slots per packed fma; fma(u, -l, a) == fma(-l, u, a)
-#pragma unroll
-            for (int q = c / 4; q < CW / 4; q++) {
-                const float4 v = ub4[q];
-                const float uu[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                for (int e = 0; e < 4; e += 2) {
-                    const int s0 = 4 * q + e;
-                    if (s0 > c) {
-#pragma unroll
-                        for (int t = 0; t < R; t++) {
-                            if (below[t]) {
-                                const float2 r2 = __ffma2_rn(make_float2(uu[e], uu[e + 1]), make_float2(-l[t], -l[t]),
-                                                             make_float2(a[t][s0], a[t][s0 + 1]));
-                                a[t][s0] = r2.x;
-                                a[t][s0 + 1] = r2.y;
-                            }
-                        }
-                    } else {
-#pragma unroll
-                        for (int h = 0; h < 2; h++) {
-                            const int sl = s0 + h;
-                            if (sl > c || (sl == c && warp > w)) {
-#pragma unroll
-                                for (int t = 0; t < R; t++)
-                                    if (below[t]) a[t][sl] = fmaf(-l[t], uu[e + h], a[t][sl]);
-                            }
-                        }
-                    }
-                }
-            }
-        }
-    }
-    return info;
-}
-
-// =============================================================================================
-// Triangular solve from factors held in shared memory (32 < n <= 128; the grouped kernel stages
-// its register-resident factors there for the right-hand sides).
-// =============================================================================================
-constexpr int kMedMaxN = 128;
-constexpr int kMedRows = kMedMaxN / 32;  // rows per lane
-
-// Solves right-hand-side column y (n values, logical order after the interchanges: the lane's
-// rows i = lane + 32 t enter with y[t] = b[rmap[i]]) with the factors held in shared memory at
-// sa (physical row p, column j at sa[p + j * ld]; logical row i is physical row rmap[i]), in the reference
-// getrs's order (trans N): unit-L forward sweep, then U backward sweep with x_j = y_j / U(j,j).
-// Run by one warp; y[t] leaves as x[lane + 32 t].
-__device__ __forceinline__ void med_solve_core(const float* sa, const int* rmap, int n, int ld, int lane,
-                                               float (&y)[kMedRows])
-{
-    int ph[kMedRows];
-#pragma unroll
-    for (int t = 0; t < kMedRows; t++) ph[t] = (lane + 32 * t < n) ? rmap[lane + 32 * t] : 0;
-#pragma unroll
-    for (int kq = 0; kq < kMedRows; kq++) {
-        for (int kl = 0; kl < 32; kl++) {
-            const int k = kq * 32 + kl;
-            if (k >= n) break;
-            const float yk = __shfl_sync(0xffffffffu, y[kq], kl);
-#pragma unroll
-            for (int t = 0; t < kMedRows; t++) {
-                const int i = lane + 32 * t;
-                if (t >= kq && i > k && i < n) y[t] = fmaf(-sa[ph[t] + k * ld], yk, y[t]);
-            }
-        }
-    }
-#pragma unroll
-    for (int kq = kMedRows - 1; kq >= 0; kq--) {
-        for (int kl = 31; kl >= 0; kl--) {
-            const int k = kq * 32 + kl;
-            if (k >= n) continue;
-            const float t0 = (lane == kl) ? y[kq] / sa[ph[kq] + k * ld] : 0.0f;
-            const float xk = __shfl_sync(0xffffffffu, t0, kl);
-#pragma unroll
-            for (int t = 0; t < kMedRows; t++) {
-                const int i = lane + 32 * t;
-                if (t <= kq) {
-                    if (i == k)
-                        y[t] = xk;
-                    else if (i < k)
-                        y[t] = fmaf(-sa[ph[t] + k * ld], xk, y[t]);
-                }
-            }
-        }
-    }
 }
 
 }  // namespace opsblas
