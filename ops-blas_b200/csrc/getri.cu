@@ -11,11 +11,14 @@
 //             lane c of a warp segment solves column c of C in registers (two rows per packed
 //             f32x2 FMA) reading L/U with broadcast 16-byte loads, and C leaves through shared
 //             memory as coalesced column stores.
-//   n  > 32 : getri_generic_kernel, thread per column of C in global memory.
+//   32 < n <= 256 : getri_block_kernel, 16 columns of C a warp in registers, panels of LU shared by the
+//             CTA (lu_solve.cuh);
+//   n  > 256 : getri_generic_kernel, thread per column of C in global memory.
 #include <cuda_runtime.h>
 
 #include "internal.h"
 #include "getri_small.cuh"
+#include "lu_solve.cuh"
 #include "small_common.cuh"
 
 namespace opsblas {
@@ -72,7 +75,101 @@ getri_small_kernel(const float* const* __restrict__ Aarray, int lda, const int* 
     if (mvalid && r == 0) info[m] = inf;
 }
 
-// n > 32: thread per column of C, the reference's column-parallel structure, in global memory.
+// 32 < n <= 256: every warp holds 16 columns of C in registers (rows over the lanes) and the CTA's
+// warps share the factors' panels, staged two deep by cp.async (lu_solve.cuh). LU is read once per CTA
+// and C written once. A zero U(j,j) ends the U sweep, as the reference's does.
+template <int R>
+__global__ void __launch_bounds__(256, R <= 4 ? 2 : 1)
+getri_block_kernel(const float* const* __restrict__ Aarray, int n, int lda, const int* __restrict__ ipiv,
+                   float* const* __restrict__ Carray, int ldc, int* __restrict__ info)
+{
+    constexpr int CW = 16;
+    constexpr int LDP = 32 * R + 4;
+    __shared__ __align__(16) float panel[2][kSvNB * LDP];
+    __shared__ __align__(16) float ubuf[8][kSvNB * kSvULd<CW>];
+    __shared__ int pv[32 * R], src[32 * R];
+    const long long m = blockIdx.x;
+    const float* A = Aarray[m];
+    const int tid = threadIdx.x, threads = blockDim.x, warp = tid >> 5, lane = tid & 31;
+    const bool vec = (reinterpret_cast<uintptr_t>(A) & 15) == 0 && (lda & 3) == 0;
+    const int nb = (n + kSvNB - 1) / kSvNB;
+    sv_stage(panel[0], LDP, A, lda, n, 0, 0, n, vec, tid, threads);
+    for (int i = tid; i < n; i += threads) pv[i] = ipiv ? ipiv[m * n + i] - 1 : i;
+    __syncthreads();
+    // src[i]: the row that the interchanges bring to position i (traced back, invalid pivots skipped)
+    for (int i = tid; i < n; i += threads) {
+        int x = i;
+#pragma unroll 4
+        for (int k = n - 1; k >= 0; k--) {
+            const int q = pv[k];
+            if ((unsigned)q < (unsigned)n && q != k) x = x == k ? q : (x == q ? k : x);
+        }
+        src[i] = x;
+    }
+    __syncthreads();
+    const int c0 = ((int)blockIdx.y * (threads >> 5) + warp) * CW;  // this warp's columns of C
+    float2 p[R][CW / 2];
+#pragma unroll
+    for (int t = 0; t < R; t++) {
+        const int one = lane + 32 * t < n ? src[lane + 32 * t] - c0 : -1;
+#pragma unroll
+        for (int h = 0; h < CW / 2; h++)
+            p[t][h] = make_float2(one == 2 * h ? 1.0f : 0.0f, one == 2 * h + 1 ? 1.0f : 0.0f);
+    }
+    float* u = ubuf[warp];
+    const bool work = c0 < n;
+    int buf = 0;
+    for (int b = 0; b < nb; b++, buf ^= 1) {
+        cp_async_wait_all();
+        __syncthreads();
+        if (b + 1 < nb)
+            sv_stage(panel[buf ^ 1], LDP, A, lda, n, (b + 1) * kSvNB, (b + 1) * kSvNB, n, vec, tid, threads);
+        else
+            sv_stage(panel[buf ^ 1], LDP, A, lda, n, b * kSvNB, 0, n, vec, tid, threads);
+        if (work) sv_forward<R, CW>(p, panel[buf], LDP, u, b * kSvNB, n, lane);
+    }
+    int inf = 0;
+    for (int b = nb - 1; b >= 0; b--, buf ^= 1) {
+        cp_async_wait_all();
+        __syncthreads();
+        const int k0 = b * kSvNB;
+        const float* P = panel[buf];
+        // the panel's highest zero on the diagonal: the same in every thread
+        const bool zero = lane < kSvNB && k0 + lane < n && P[k0 + lane + lane * LDP] == 0.0f;
+        const unsigned zeros = __ballot_sync(0xffffffffu, zero);
+        const int stop = zeros ? k0 + 31 - __clz(zeros) : -1;
+        if (b > 0 && stop < 0)
+            sv_stage(panel[buf ^ 1], LDP, A, lda, n, k0 - kSvNB, 0, k0, vec, tid, threads);
+        if (work) sv_backward<R, CW>(p, P, LDP, u, k0, n, stop, lane);
+        if (stop >= 0) {
+            inf = stop + 1;
+            break;
+        }
+    }
+    float* C = Carray[m];
+#pragma unroll
+    for (int c = 0; c < CW; c++) {
+        if (c0 + c < n) {
+            float* col = C + (long long)(c0 + c) * ldc;
+#pragma unroll
+            for (int t = 0; t < R; t++)
+                if (lane + 32 * t < n) col[lane + 32 * t] = (c & 1) ? p[t][c / 2].y : p[t][c / 2].x;
+        }
+    }
+    if (blockIdx.y == 0 && tid == 0) info[m] = inf;
+}
+
+template <int R>
+static void launch_getri_block(cudaStream_t st, const float* const* Aarray, int n, int lda, const int* ipiv,
+                               float* const* Carray, int ldc, int* info, int batch)
+{
+    const int blocks = (n + 15) / 16;                 // warps' worth of columns
+    const int parts = (blocks + 7) / 8, warps = (blocks + parts - 1) / parts;
+    getri_block_kernel<R><<<dim3((unsigned)batch, (unsigned)parts), warps * 32, 0, st>>>(Aarray, n, lda, ipiv, Carray,
+                                                                                        ldc, info);
+}
+
+// n > 256: thread per column of C, the reference's column-parallel structure, in global memory.
 // Several CTAs share one matrix along the columns (grid.y).
 constexpr int kGenericThreads = 256;
 
@@ -182,6 +279,16 @@ extern "C" aclblasStatus_t aclblasSgetriBatched(
             default:
                 break;
         }
+    } else if (n <= 64) {
+        launch_getri_block<2>(st, Aarray, n, lda, PivotArray, Carray, ldc, infoArray, batchSize);
+    } else if (n <= 96) {
+        launch_getri_block<3>(st, Aarray, n, lda, PivotArray, Carray, ldc, infoArray, batchSize);
+    } else if (n <= 128) {
+        launch_getri_block<4>(st, Aarray, n, lda, PivotArray, Carray, ldc, infoArray, batchSize);
+    } else if (n <= 192) {
+        launch_getri_block<6>(st, Aarray, n, lda, PivotArray, Carray, ldc, infoArray, batchSize);
+    } else if (n <= 256) {
+        launch_getri_block<8>(st, Aarray, n, lda, PivotArray, Carray, ldc, infoArray, batchSize);
     } else {
         dim3 grid((unsigned)batchSize, (unsigned)((n + kGenericThreads - 1) / kGenericThreads));
         getri_generic_kernel<<<grid, kGenericThreads, 0, st>>>(Aarray, n, lda, PivotArray, Carray, ldc, infoArray);
