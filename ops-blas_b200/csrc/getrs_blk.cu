@@ -1,4 +1,4 @@
-// aclblasSgetrsBatched, trans N, n > 32: one CTA per matrix, blocked substitution with the
+// aclblasSgetrsBatched, trans N, n > 128: one CTA per matrix, blocked substitution with the
 // right-hand sides resident in shared memory.
 //
 // The reference solve (sgetrs_batched_kernel.cpp:83-200) is laswp, then the unit-L forward sweep

@@ -73,17 +73,18 @@ inline int max1(int n) { return n > 1 ? n : 1; }
 // pass NULL for converged matrices).
 cudaError_t getrs_launch(cudaStream_t st, bool trans, int n, int nrhs, const float* const* Aarray, int lda,
                          const int* devIpiv, float* const* Barray, int ldb, int batchCount);
-// getrs_blk.cu: trans N, n > 32, blocked substitution with the right-hand sides in shared memory.
+// getrs_blk.cu: trans N, n > 128, blocked substitution with the right-hand sides in shared memory.
 bool getrs_blk_supported(int n);
 cudaError_t getrs_blk_launch(cudaStream_t st, int n, int nrhs, const float* const* Aarray, int lda, const int* ipiv,
                              float* const* Barray, int ldb, int batch);
-// getrs_trhs.cu: trans T / C, n > 32, one thread per right-hand side (reference order).
+// getrs_trhs.cu: trans T / C, n > 128, one thread per right-hand side (reference order).
 bool getrs_trhs_supported(int n);
 cudaError_t getrs_trhs_launch(cudaStream_t st, int n, int nrhs, const float* const* Aarray, int lda, const int* ipiv,
                               float* const* Barray, int ldb, int batch);
-bool getrs_nrhs_preferred(int n, int nrhs, int batch);
-cudaError_t getrs_nrhs_launch(cudaStream_t st, int n, int nrhs, const float* const* Aarray, int lda, const int* ipiv,
-                              float* const* Barray, int ldb, int batch);
+// getrs_staged.cu: 32 < n <= 128, LU in shared memory, one thread per right-hand side.
+bool getrs_staged_supported(int n);
+cudaError_t getrs_staged_launch(cudaStream_t st, bool trans, int n, int nrhs, const float* const* Aarray, int lda,
+                                const int* ipiv, float* const* Barray, int ldb, int batch);
 // Element types of the batched GEMMs' operands in global memory.
 enum class GemmElem { F32, F16, BF16, E4M3, E5M2 };
 

@@ -16,37 +16,10 @@
 
 #include <cuda_runtime.h>
 
+#include "f32x2.cuh"
 #include "small_common.cuh"
 
 namespace opsblas {
-
-// Two packed floats, the operand of the f32x2 instructions.
-using f32x2 = unsigned long long;
-
-__device__ __forceinline__ f32x2 f2_pack(float x, float y)
-{
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-    return r;
-}
-__device__ __forceinline__ f32x2 f2_dup(float x) { return f2_pack(x, x); }
-__device__ __forceinline__ void f2_unpack(f32x2 v, float& x, float& y)
-{
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
-}
-__device__ __forceinline__ float f2_get(f32x2 v, int i)
-{
-    float x, y;
-    f2_unpack(v, x, y);
-    return i ? y : x;
-}
-// each half an IEEE fma
-__device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c)
-{
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
 
 constexpr int kMidNB = 16;    // columns of a block
 constexpr int kMidULd = 20;   // row stride of the update's U rows (16-byte rows, conflict-free by eights)

@@ -89,3 +89,28 @@ def test_getri_block_edges(handle, n):
     oc = np.full((batch, n, ldc), -7.0, np.float32)
     oinfo = O.port_getri(lu, n, lda, None, oc, ldc)
     assert_bitwise(c, oc, f"C n={n} without pivots")
+
+
+@pytest.mark.parametrize("n", [33, 40, 63, 64, 65, 72, 96, 97, 104, 127, 128])
+@pytest.mark.parametrize("trans", ["N", "T"])
+def test_getrs_staged_edges(handle, n, trans):
+    """The staged solve (getrs_staged.cu): block and tile edges, column counts on both sides of its warp and CTA
+    limits, odd strides, invalid pivots, zeros, infinities and NaN in the right-hand sides."""
+    rng = np.random.default_rng(n)
+    for nrhs, batch, pad in ((1, 5, 0), (2, 3, 1), (3, 37, 0), (8, 9, 4), (17, 2, 0), (33, 2, 3), (130, 1, 0)):
+        ld = n + pad
+        lu = rng.standard_normal((batch, n, ld)).astype(np.float32)
+        piv, _, _ = O.port_getrf(lu, n, ld)
+        piv[0, 0] = 0
+        piv[0, n - 1] = n + 7
+        b = rng.standard_normal((batch, nrhs, ld)).astype(np.float32)
+        b[0, 0, : n // 2] = 0.0
+        if nrhs > 2:
+            b[batch - 1, 1, n - 1] = np.inf
+            b[batch - 1, 2, 0] = np.nan
+        want = b.copy()
+        with np.errstate(all="ignore"):
+            O.port_getrs(trans, lu, n, ld, piv, want, nrhs, ld)
+        B = to_dev(b, "cuda")
+        handle.getrs(trans, to_dev(lu, "cuda"), n, ld, to_dev(piv, "cuda"), B, nrhs, ld)
+        assert_bitwise(to_host(B), want, f"n={n} nrhs={nrhs} {trans}")
