@@ -32,7 +32,8 @@ __device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c)
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
-// Each half rounded on its own; .rn keeps a product and a sum from being joined into an fma.
+// Each half rounded on its own. (A product that feeds a packed sum directly is joined with it into an fma
+// all the same: negate it in between where both roundings are wanted.)
 __device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b)
 {
     f32x2 r;

@@ -12,16 +12,19 @@
 //   M <  N: LQ by row reflectors, forward substitution L y = c (same stop rule), rows M..N-1 of C
 //           zeroed, Q^T applied in reverse reflector order.
 // info is per matrix (device array), as the reference kernel writes it (its CPU golden keeps one
-// value for the batch). Small QR-path systems run a warp per system (gels_warp_kernel); the rest
-// one CTA per matrix: thread 0 forms each reflector, threads take the independent columns / rows /
+// value for the batch). Small QR-path systems run a warp per system (gels_warp_kernel), larger ones
+// that fit shared memory a CTA each (gels_smem_kernel); the rest one CTA per matrix in global memory: thread 0 forms each reflector, threads take the independent columns / rows /
 // right-hand sides of every step. Every sum runs in index order with each product rounded before
 // it is added -- bit for bit the CPU oracle's restatement, on both paths.
 // Parity with the reference is its tests' rule (MERE_MARE on the solution against LAPACK sgels_).
 #include <cuda_runtime.h>
 
+#include <cstdint>
 #include <utility>
 
 #include "internal.h"
+#include "qr_col.cuh"
+#include "qr_smem.cuh"
 #include "small_common.cuh"
 
 namespace opsblas {
@@ -209,18 +212,12 @@ gels_kernel(int trans, int m, int n, int nrhs, float* const* __restrict__ Aarray
 constexpr int kGelsWarps = 4;
 
 template <int M, int K>
-__device__ __forceinline__ void gels_warp_step(float (&col)[M], float* vb, int lane, int ncols, float& tau_k)
+__device__ __forceinline__ void gels_warp_step(QrCol<M>& col, float* vb, int lane, int ncols)
 {
     // xnorm = ||A(K+1:, K)||, row order, formed by every lane for its own column (lane K's is used)
-    float ss = 0.0f;
-#pragma unroll
-    for (int r = K + 1; r < M; r++) ss = __fadd_rn(ss, __fmul_rn(col[r], col[r]));
-    const float xnorm = sqrtf(__shfl_sync(0xffffffffu, ss, K));
-    const float akk = __shfl_sync(0xffffffffu, col[K], K);
-    if (xnorm < 1.0e-30f && akk >= 0.0f) {
-        tau_k = 0.0f;
-        return;  // uniform
-    }
+    const float xnorm = sqrtf(__shfl_sync(0xffffffffu, qc_dot<M, K + 1>(0.0f, col, col), K));
+    const float akk = __shfl_sync(0xffffffffu, qc_get<M>(col, K), K);
+    if (xnorm < 1.0e-30f && akk >= 0.0f) return;  // uniform: no reflector
     const float na = fabsf(akk);
     const float sc = na > xnorm ? na : xnorm;
     const float sa = __fdiv_rn(akk, sc), sx = __fdiv_rn(xnorm, sc);
@@ -228,35 +225,37 @@ __device__ __forceinline__ void gels_warp_step(float (&col)[M], float* vb, int l
     const float beta = akk >= 0.0f ? -nm : nm;
     const float t = __fdiv_rn(__fsub_rn(beta, akk), beta);
     const float scalev = __fdiv_rn(1.0f, __fsub_rn(akk, beta));
-    tau_k = t;
     if (lane == K) {
-        col[K] = beta;
-#pragma unroll
-        for (int r = K + 1; r < M; r++) {
-            col[r] = __fmul_rn(col[r], scalev);
-            vb[r] = col[r];
+        if (K & 1) {
+            qc_set<M>(col, K, beta);
+        } else {
+            float a, b;
+            f2_unpack(col[K / 2], a, b);
+            col[K / 2] = f2_pack(beta, __fmul_rn(b, scalev));
         }
+        const f32x2 ss = f2_dup(scalev);
+#pragma unroll
+        for (int h = (K + 2) / 2; h < (M + 1) / 2; h++) col[h] = f2_mul(col[h], ss);
+        qc_put<M, K + 1>(vb, col);
     }
     __syncwarp();
     if (lane > K && lane < ncols) {
-        // w = v . a + a(K); a(K) -= t w; a += (-t w) v
-        float w = 0.0f;
-#pragma unroll
-        for (int r = K + 1; r < M; r++) w = __fadd_rn(w, __fmul_rn(vb[r], col[r]));
-        w = __fadd_rn(w, col[K]);
-        col[K] = __fsub_rn(col[K], __fmul_rn(t, w));
-        const float alpha = -__fmul_rn(t, w);
-#pragma unroll
-        for (int r = K + 1; r < M; r++) col[r] = __fadd_rn(col[r], __fmul_rn(alpha, vb[r]));
+        // w = v . a + a(K); a(K) -= t w; a -= (t w) v
+        QrCol<M> v;
+        qc_take<M, K + 1>(v, vb);
+        const float head = qc_get<M>(col, K);
+        const float tw = __fmul_rn(t, __fadd_rn(qc_dot<M, K + 1>(0.0f, v, col), head));
+        qc_axmy<M, K + 1>(col, v, tw);
+        qc_set<M>(col, K, __fsub_rn(head, tw));
     }
     __syncwarp();  // v read before the next reflector writes it
 }
 
 template <int M, int... K>
-__device__ __forceinline__ void gels_warp_all(float (&col)[M], float* vb, int lane, int ncols, int N, float* tau,
+__device__ __forceinline__ void gels_warp_all(QrCol<M>& col, float* vb, int lane, int ncols, int N,
                                               std::integer_sequence<int, K...>)
 {
-    ((K < N ? gels_warp_step<M, K>(col, vb, lane, ncols, tau[K]) : void()), ...);
+    ((K < N ? gels_warp_step<M, K>(col, vb, lane, ncols) : void()), ...);
 }
 
 template <int M>
@@ -264,7 +263,7 @@ __global__ void __launch_bounds__(kGelsWarps * 32)
 gels_warp_kernel(int trans, int m, int n, int nrhs, float* const* __restrict__ Aarray, int lda,
                  float* const* __restrict__ Carray, int ldc, int* __restrict__ info, int batch)
 {
-    __shared__ float vbuf[kGelsWarps][32];
+    __shared__ __align__(16) float vbuf[kGelsWarps][32];
     __shared__ float rbuf[kGelsWarps][32 * 33];  // R (N x N), column c at rbuf[c * 33]
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -274,66 +273,126 @@ gels_warp_kernel(int trans, int m, int n, int nrhs, float* const* __restrict__ A
     float* C = Carray[b];
     const int N = trans ? m : n;  // effective columns (M = effective rows)
     const int ncols = N + nrhs;
-    float col[M];
-    if (lane < N) {
+    const bool veca = (lda & 3) == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;
+    const bool vecc = (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
+    QrCol<M> col;
+    if (lane < N && trans) {
 #pragma unroll
-        for (int r = 0; r < M; r++) col[r] = trans ? A[lane + (long long)r * lda] : A[r + (long long)lane * lda];
+        for (int h = 0; h < (M + 1) / 2; h++)
+            col[h] = f2_pack(A[lane + (long long)(2 * h) * lda], 2 * h + 1 < M ? A[lane + (long long)(2 * h + 1) * lda] : 0.0f);
+    } else if (lane < N) {
+        qc_load<M>(col, A + (long long)lane * lda, veca);
     } else if (lane < ncols) {
-        const float* c = C + (long long)(lane - N) * ldc;
-#pragma unroll
-        for (int r = 0; r < M; r++) col[r] = c[r];
+        qc_load<M>(col, C + (long long)(lane - N) * ldc, vecc);
     } else {
 #pragma unroll
-        for (int r = 0; r < M; r++) col[r] = 0.0f;
+        for (int h = 0; h < (M + 1) / 2; h++) col[h] = 0ull;
     }
-    float tau[32];
-    gels_warp_all<M>(col, vbuf[warp], lane, ncols, N, tau, std::make_integer_sequence<int, M>{});
+    gels_warp_all<M>(col, vbuf[warp], lane, ncols, N, std::make_integer_sequence<int, M>{});
     // factors back (trans: the n x m transpose with leading dimension n, as the reference leaves it)
+    if (trans) __syncwarp();  // every lane has read its row of A before any lane writes the transpose
     if (lane < N) {
-        if (trans) {
-            __syncwarp();  // every lane has read its row of A before any lane writes the transpose
-#pragma unroll
-            for (int r = 0; r < M; r++) A[r + (long long)lane * M] = col[r];
-        } else {
-#pragma unroll
-            for (int r = 0; r < M; r++) A[r + (long long)lane * lda] = col[r];
-        }
-    } else if (trans) {
-        __syncwarp();
+        if (trans)
+            qc_store<M>(col, A + (long long)lane * M, M % 4 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0);
+        else
+            qc_store<M>(col, A + (long long)lane * lda, veca);
     }
     // R to shared memory; the highest zero diagonal stops the first right-hand side there
     float* R = rbuf[warp];
     if (lane < N) {
 #pragma unroll
         for (int r = 0; r < M; r++)
-            if (r < N) R[lane * 33 + r] = col[r];
+            if (r < N) R[lane * 33 + r] = qc_get<M>(col, r);
     }
     __syncwarp();
-    int stop = -1;
-    for (int i = N - 1; i >= 0; i--)
-        if (R[i * 33 + i] == 0.0f) {
-            stop = i;
-            break;
-        }
+    const unsigned zeros = __ballot_sync(0xffffffffu, lane < N && R[lane * 33 + lane] == 0.0f);
+    const int stop = zeros ? 31 - __clz(zeros) : -1;
     const int j = lane - N;
-    if (j >= 0 && j < (stop >= 0 ? 1 : nrhs)) {
+    if (j >= 0 && j < nrhs) {
+        float x[M];
 #pragma unroll
-        for (int i = M - 1; i >= 0; i--) {
-            if (i < N && i > stop) {
-                float sum = 0.0f;
+        for (int r = 0; r < M; r++) x[r] = qc_get<M>(col, r);
+        if (j < (stop >= 0 ? 1 : nrhs)) {
 #pragma unroll
-                for (int q = i + 1; q < M; q++)
-                    if (q < N) sum = __fadd_rn(sum, __fmul_rn(R[q * 33 + i], col[q]));
-                col[i] = __fdiv_rn(__fsub_rn(col[i], sum), R[i * 33 + i]);
+            for (int i = M - 1; i >= 0; i--) {
+                if (i < N && i > stop) {
+                    float sum = 0.0f;
+#pragma unroll
+                    for (int q = i + 1; q < M; q++)
+                        if (q < N) sum = __fadd_rn(sum, __fmul_rn(R[q * 33 + i], x[q]));
+                    x[i] = __fdiv_rn(__fsub_rn(x[i], sum), R[i * 33 + i]);
+                }
             }
         }
-    }
-    if (j >= 0 && j < nrhs) {
-        float* c = C + (long long)j * ldc;
 #pragma unroll
-        for (int r = 0; r < M; r++) c[r] = col[r];
+        for (int h = 0; h < (M + 1) / 2; h++) col[h] = f2_pack(x[2 * h], 2 * h + 1 < M ? x[2 * h + 1 < M ? 2 * h + 1 : 0] : 0.0f);
+        qc_store<M>(col, C + (long long)j * ldc, vecc);
     }
     if (lane == 0) info[b] = stop >= 0 ? stop + 1 : 0;
+}
+
+// QR-path systems beyond the warp kernel that fit shared memory: one a CTA, a warp per 64 columns, the
+// right-hand sides as further columns (qr_smem.cuh), then a thread per right-hand side for R x = c.
+// 48 x 30 with 4 right-hand sides x 4096: 1031 us in global memory, 202 here; 40 x 10, 2 x 8192: 349, 128.
+__global__ void __launch_bounds__(128)
+gels_smem_kernel(int trans, int m, int n, int nrhs, float* const* __restrict__ Aarray, int lda,
+                 float* const* __restrict__ Carray, int ldc, int* __restrict__ info)
+{
+    extern __shared__ __align__(16) float dyn[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+    const int rows = trans ? n : m, N = trans ? m : n, cols = N + nrhs;
+    const QsSmem M(dyn, rows, cols);
+    float* A = Aarray[blockIdx.x];
+    float* C = Carray[blockIdx.x];
+    if (trans) {
+        for (int r = warp; r < rows; r += warps)
+            for (int c = lane; c < N; c += 32) M.a[r * M.ld + c] = A[c + (long long)r * lda];
+    } else {
+        for (int c = warp; c < N; c += warps)
+#pragma unroll 4
+            for (int r = lane; r < rows; r += 32) M.a[r * M.ld + c] = A[r + (long long)c * lda];
+    }
+    for (int j = warp; j < nrhs; j += warps)
+        for (int r = lane; r < rows; r += 32) M.a[r * M.ld + N + j] = C[r + (long long)j * ldc];
+    qs_sync(warps);
+    qs_factor<true>(
+        M, rows, N, cols, warps, tid,
+        [](float ss, float akk, float& t, float& beta, float& scalev) {
+            const float xnorm = sqrtf(ss);
+            if (xnorm < 1.0e-30f && akk >= 0.0f) return false;
+            const float na = fabsf(akk);
+            const float sc = na > xnorm ? na : xnorm;
+            const float sa = __fdiv_rn(akk, sc), sx = __fdiv_rn(xnorm, sc);
+            const float nm = __fmul_rn(sc, sqrtf(__fadd_rn(__fmul_rn(sa, sa), __fmul_rn(sx, sx))));
+            beta = akk >= 0.0f ? -nm : nm;
+            t = __fdiv_rn(__fsub_rn(beta, akk), beta);
+            scalev = __fdiv_rn(1.0f, __fsub_rn(akk, beta));
+            return true;
+        },
+        [](float x, float sc) { return __fmul_rn(x, sc); }, [](int, float) {});
+    // factors back (trans: the n x m transpose with leading dimension n, as the reference leaves it)
+    const int ldo = trans ? rows : lda;
+    for (int c = warp; c < N; c += warps)
+#pragma unroll 4
+        for (int r = lane; r < rows; r += 32) A[r + (long long)c * ldo] = M.a[r * M.ld + c];
+    // the highest zero diagonal stops the first right-hand side there and leaves the others
+    int stop = -1;
+    for (int i = N - 1; i >= 0 && stop < 0; i--)
+        if (M.a[i * M.ld + i] == 0.0f) stop = i;
+    for (int j = tid; j < (stop >= 0 ? 1 : nrhs); j += warps * 32) {
+        float* c = M.a + N + j;
+        for (int i = N - 1; i > stop; i--) {
+            const float* row = M.a + i * M.ld;
+            float sum = 0.0f;
+#pragma unroll 4
+            for (int q = i + 1; q < N; q++) sum = __fadd_rn(sum, __fmul_rn(row[q], c[q * M.ld]));
+            c[i * M.ld] = __fdiv_rn(__fsub_rn(c[i * M.ld], sum), row[i]);
+        }
+    }
+    qs_sync(warps);
+    for (int j = warp; j < nrhs; j += warps)
+        for (int r = lane; r < rows; r += 32) C[r + (long long)j * ldc] = M.a[r * M.ld + N + j];
+    if (tid == 0) info[blockIdx.x] = stop >= 0 ? stop + 1 : 0;
 }
 
 size_t gels_smem_bytes(int trans, int m, int n, int lda)
@@ -404,6 +463,13 @@ extern "C" aclblasStatus_t aclblasSgelsBatched(aclblasHandle_t handle, aclblasOp
         log_error(kApi, "the transposed solve needs lda*n <= %zu floats of shared memory, got lda=%d n=%d",
                   kGelsMaxSmem / 4, lda, n);
         return ACLBLAS_STATUS_NOT_SUPPORTED;
+    }
+    if (effM >= effN && qs_supported(effM, effN + nrhs)) {
+        const cudaError_t e = ensure_smem_limit(gels_smem_kernel, kQsMaxBytes);
+        if (e != cudaSuccess) return launch_status(kApi, e);
+        gels_smem_kernel<<<(unsigned)batchSize, qs_warps(effN + nrhs) * 32, qs_bytes(effM, effN + nrhs),
+                           handle->stream>>>(t, m, n, nrhs, Aarray, lda, Carray, ldc, devInfo);
+        return launch_status(kApi, cudaGetLastError());
     }
     const cudaError_t e = ensure_smem_limit(gels_kernel, (int)kGelsMaxSmem);
     if (e != cudaSuccess) return launch_status(kApi, e);

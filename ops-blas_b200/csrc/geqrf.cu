@@ -13,31 +13,33 @@
 //   m, n <= 32 : geqrf_col_kernel<M>, one warp per matrix, lane c = column c in registers (every
 //                sum local, in row order), the reflector published through shared memory with
 //                its divisions one row per lane, the column update in packed f32x2 operations;
+//   n <= 256 and the matrix in shared memory: geqrf_smem_kernel, a warp per 64 columns;
 //   otherwise  : geqrf_generic_kernel, one CTA per matrix in global memory (correctness path):
 //                thread 0 forms the reflector, thread t updates columns i+1+t, i+1+t+256, ...
 #include <cuda_runtime.h>
 
+#include <cstdint>
 #include <utility>
 
 #include "internal.h"
+#include "qr_col.cuh"
+#include "qr_smem.cuh"
 #include "small_common.cuh"
 
 namespace opsblas {
 
 constexpr int kQrWarps = 8;
 
-// Reflector I of the warp's matrix. Lane c holds column c (rows in registers, M = m rows); every
-// sum runs locally in row order, so the arithmetic is the row-order restatement's. The reflector's
-// divisions are shared out one row per lane through the warp's shared-memory column buffer.
+// Reflector I of the warp's matrix. Lane c holds column c; every sum runs locally in row order, so the
+// arithmetic is the row-order restatement's. The reflector's divisions are shared out one row per lane
+// through the warp's shared-memory column buffer. Packed pairs and 16-byte column loads: 32 x 32 x 65536
+// 971 -> 545 us, 24 x 17 x 32768 174 -> 125 us.
 template <int M, int I>
-__device__ __forceinline__ void qr_col_step(float (&col)[M], float& mytau, float* vb, int lane, int n)
+__device__ __forceinline__ void qr_col_step(QrCol<M>& col, float& mytau, float* vb, int lane, int n)
 {
     // sigma = sum_{r>I} A(r,I)^2 (every lane forms it for its own column; lane I's is used)
-    float sigma = 0.0f;
-#pragma unroll
-    for (int r = I + 1; r < M; r++) sigma = __fadd_rn(sigma, __fmul_rn(col[r], col[r]));
-    sigma = __shfl_sync(0xffffffffu, sigma, I);
-    const float x1 = __shfl_sync(0xffffffffu, col[I], I);
+    const float sigma = __shfl_sync(0xffffffffu, qc_dot<M, I + 1>(0.0f, col, col), I);
+    const float x1 = __shfl_sync(0xffffffffu, qc_get<M>(col, I), I);
     float t, alpha;
     if (sigma == 0.0f) {
         t = 0.0f;
@@ -51,44 +53,31 @@ __device__ __forceinline__ void qr_col_step(float (&col)[M], float& mytau, float
     if (t == 0.0f) return;  // uniform: A(I,I) stays x1 == alpha, no update
     const float vscale = __fsub_rn(x1, alpha);
     // v_r = A(r,I) / vscale for r > I: lane I publishes its column, lane r divides row r
-    if (lane == I) {
-#pragma unroll
-        for (int r = I + 1; r < M; r++) vb[r] = col[r];
-    }
+    if (lane == I) qc_put<M, I + 1>(vb, col);
     __syncwarp();
     if (lane > I && lane < M) vb[lane] = __fdiv_rn(vb[lane], vscale);
     __syncwarp();
-    float v[M];
-#pragma unroll
-    for (int r = I + 1; r < M; r++) v[r] = vb[r];
+    QrCol<M> v;
+    qc_take<M, I + 1>(v, vb);
     if (lane == I) {
-        col[I] = alpha;
+        const float above = I & 1 ? qc_get<M>(col, I - 1 > 0 ? I - 1 : 0) : 0.0f;  // shares I's pair
 #pragma unroll
-        for (int r = I + 1; r < M; r++) col[r] = v[r];
+        for (int h = (I + 2) / 2; h < (M + 1) / 2; h++) col[h] = v[h];
+        col[I / 2] = I & 1 ? f2_pack(above, alpha)
+                           : f2_pack(alpha, I + 1 < M ? qc_get<M>(v, I + 1 < M ? I + 1 : 0) : 0.0f);
     } else if (lane > I && lane < n) {
         // dot = A(I,c) + sum_{r>I} v_r A(r,c) in row order, then A(r,c) -= coef v_r, A(I,c) -= coef
-        float dot = col[I];
-#pragma unroll
-        for (int r = I + 1; r < M; r++) dot = __fadd_rn(dot, __fmul_rn(v[r], col[r]));
-        const float coef = __fmul_rn(t, dot);
-        const float2 cc = make_float2(coef, coef);
-        int r = I + 1;
-#pragma unroll
-        for (; r + 1 < M; r += 2) {
-            const float2 p = __fmul2_rn(cc, make_float2(v[r], v[r + 1]));
-            const float2 q = __fadd2_rn(make_float2(col[r], col[r + 1]), make_float2(-p.x, -p.y));
-            col[r] = q.x;
-            col[r + 1] = q.y;
-        }
-        if (r < M) col[r] = __fsub_rn(col[r], __fmul_rn(coef, v[r]));
-        col[I] = __fsub_rn(col[I], coef);
+        const float head = qc_get<M>(col, I);
+        const float coef = __fmul_rn(t, qc_dot<M, I + 1>(head, v, col));
+        qc_axmy<M, I + 1>(col, v, coef);
+        qc_set<M>(col, I, __fsub_rn(head, coef));
     }
     __syncwarp();  // the buffer is read before the next reflector writes it
 }
 
 // Reflectors 0 .. min(m, n) - 1, one instantiation per row index.
 template <int M, int... I>
-__device__ __forceinline__ void qr_col_all(float (&col)[M], float& mytau, float* vb, int lane, int n,
+__device__ __forceinline__ void qr_col_all(QrCol<M>& col, float& mytau, float* vb, int lane, int n,
                                            std::integer_sequence<int, I...>)
 {
     ((I < n ? qr_col_step<M, I>(col, mytau, vb, lane, n) : void()), ...);
@@ -98,7 +87,7 @@ template <int M>
 __global__ void __launch_bounds__(kQrWarps * 32)
 geqrf_col_kernel(float* const* __restrict__ Aarray, int n, int lda, float* const* __restrict__ TauArray, int batch)
 {
-    __shared__ float vbuf[kQrWarps][32];
+    __shared__ __align__(16) float vbuf[kQrWarps][32];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const long long b = (long long)blockIdx.x * kQrWarps + warp;
@@ -106,18 +95,50 @@ geqrf_col_kernel(float* const* __restrict__ Aarray, int n, int lda, float* const
     float* A = Aarray[b];
     float* tau = TauArray[b];
     const bool cv = lane < n;
-    float col[M];
-    const float* Ac = A + (long long)lane * lda;
+    const bool vec = (lda & 3) == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;
+    QrCol<M> col;
+    float* Ac = A + (long long)lane * lda;
+    if (cv) {
+        qc_load<M>(col, Ac, vec);
+    } else {
 #pragma unroll
-    for (int r = 0; r < M; r++) col[r] = cv ? Ac[r] : 0.0f;
+        for (int h = 0; h < (M + 1) / 2; h++) col[h] = 0ull;
+    }
     float mytau = 0.0f;
     qr_col_all<M>(col, mytau, vbuf[warp], lane, n, std::make_integer_sequence<int, M>{});
-    if (cv) {
-        float* Aw = A + (long long)lane * lda;
-#pragma unroll
-        for (int r = 0; r < M; r++) Aw[r] = col[r];
-    }
+    if (cv) qc_store<M>(col, Ac, vec);
     if (lane < M && lane < n) tau[lane] = mytau;
+}
+
+// Larger shapes that fit shared memory: one matrix a CTA, a warp per 64 columns (qr_smem.cuh). Bound by
+// instruction issue and the row-order sums. 64 x 48 x 4096: 377 us, the generic kernel's thread-0
+// reflector over global memory 3550; 40 x 33 x 4096: 156 and 550; 200 x 200 x 148: 912 and 3680.
+__global__ void __launch_bounds__(128)
+geqrf_smem_kernel(float* const* __restrict__ Aarray, int m, int n, int lda, float* const* __restrict__ TauArray)
+{
+    extern __shared__ __align__(16) float dyn[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+    const QsSmem M(dyn, m, n);
+    float* A = Aarray[blockIdx.x];
+    float* tau = TauArray[blockIdx.x];
+    for (int c = warp; c < n; c += warps)
+#pragma unroll 4
+        for (int r = lane; r < m; r += 32) M.a[r * M.ld + c] = A[r + (long long)c * lda];
+    qs_sync(warps);
+    qs_factor<false>(
+        M, m, m < n ? m : n, n, warps, tid,
+        [](float sigma, float x1, float& t, float& alpha, float& sc) {
+            if (sigma == 0.0f) return false;
+            const float normx = sqrtf(__fadd_rn(sigma, __fmul_rn(x1, x1)));
+            alpha = x1 >= 0.0f ? -normx : normx;
+            t = __fdiv_rn(__fsub_rn(alpha, x1), alpha);
+            sc = __fsub_rn(x1, alpha);
+            return t != 0.0f;
+        },
+        [](float x, float sc) { return __fdiv_rn(x, sc); }, [&](int i, float t) { tau[i] = t; });
+    for (int c = warp; c < n; c += warps)
+#pragma unroll 4
+        for (int r = lane; r < m; r += 32) A[r + (long long)c * lda] = M.a[r * M.ld + c];
 }
 
 constexpr int kQrThreads = 256;
@@ -235,6 +256,10 @@ extern "C" aclblasStatus_t aclblasSgeqrfBatched(aclblasHandle_t handle, int m, i
             default:
                 break;
         }
+    } else if (qs_supported(m, n)) {
+        const cudaError_t e = ensure_smem_limit(geqrf_smem_kernel, kQsMaxBytes);
+        if (e != cudaSuccess) return launch_status(kApi, e);
+        geqrf_smem_kernel<<<(unsigned)batchSize, qs_warps(n) * 32, qs_bytes(m, n), st>>>(Aarray, m, n, lda, TauArray);
     } else {
         geqrf_generic_kernel<<<(unsigned)batchSize, kQrThreads, 0, st>>>(Aarray, m, n, lda, TauArray);
     }
