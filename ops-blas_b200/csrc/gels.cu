@@ -264,7 +264,7 @@ gels_warp_kernel(int trans, int m, int n, int nrhs, float* const* __restrict__ A
                  float* const* __restrict__ Carray, int ldc, int* __restrict__ info, int batch)
 {
     __shared__ __align__(16) float vbuf[kGelsWarps][32];
-    __shared__ float rbuf[kGelsWarps][32 * 33];  // R (N x N), column c at rbuf[c * 33]
+    __shared__ float rbuf[kGelsWarps][32 * 33];  // R (N x N) and the right-hand sides, column c at rbuf[c * 33]
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const long long b = (long long)blockIdx.x * kGelsWarps + warp;
@@ -307,25 +307,25 @@ gels_warp_kernel(int trans, int m, int n, int nrhs, float* const* __restrict__ A
     __syncwarp();
     const unsigned zeros = __ballot_sync(0xffffffffu, lane < N && R[lane * 33 + lane] == 0.0f);
     const int stop = zeros ? 31 - __clz(zeros) : -1;
+    // R x = c by a loop of N steps over shared memory (unrolled over M it ran M / N times too long)
     const int j = lane - N;
     if (j >= 0 && j < nrhs) {
-        float x[M];
+        float* x = R + lane * 33;
 #pragma unroll
-        for (int r = 0; r < M; r++) x[r] = qc_get<M>(col, r);
+        for (int r = 0; r < M; r++)
+            if (r < N) x[r] = qc_get<M>(col, r);
         if (j < (stop >= 0 ? 1 : nrhs)) {
-#pragma unroll
-            for (int i = M - 1; i >= 0; i--) {
-                if (i < N && i > stop) {
-                    float sum = 0.0f;
-#pragma unroll
-                    for (int q = i + 1; q < M; q++)
-                        if (q < N) sum = __fadd_rn(sum, __fmul_rn(R[q * 33 + i], x[q]));
-                    x[i] = __fdiv_rn(__fsub_rn(x[i], sum), R[i * 33 + i]);
-                }
+            for (int i = N - 1; i > stop; i--) {
+                const float* p = R + (i + 1) * 33 + i;
+                float sum = 0.0f;
+#pragma unroll 4
+                for (int q = i + 1; q < N; q++, p += 33) sum = __fadd_rn(sum, __fmul_rn(*p, x[q]));
+                x[i] = __fdiv_rn(__fsub_rn(x[i], sum), R[i * 33 + i]);
             }
         }
 #pragma unroll
-        for (int h = 0; h < (M + 1) / 2; h++) col[h] = f2_pack(x[2 * h], 2 * h + 1 < M ? x[2 * h + 1 < M ? 2 * h + 1 : 0] : 0.0f);
+        for (int r = 0; r < M; r++)
+            if (r < N) qc_set<M>(col, r, x[r]);
         qc_store<M>(col, C + (long long)j * ldc, vecc);
     }
     if (lane == 0) info[b] = stop >= 0 ? stop + 1 : 0;
