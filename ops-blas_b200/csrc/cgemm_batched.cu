@@ -9,18 +9,19 @@
 // CTA owns a 64 x 64 complex tile and walks k in slices of 8, staging op(A) and op(B) slices in
 // shared memory as separate real and imaginary planes (the de-interleave, conjugation for op C
 // included, happens on the load; the next slice is fetched into registers during the multiply and
-// stored into the second of two stages), keeps the four sums of its 4 x 4 complex outputs per
+// stored into the second of two stages), keeps the four sums of its 8 x 4 complex outputs per
 // thread in registers (one fmaf per product, k in order), and applies the combine in the
 // reference's operation order in the epilogue. No workspace, one launch, C read once (only when
 // beta != 0) and written once.
 #include <climits>
 #include <cuda_runtime.h>
 
+#include "f32x2.cuh"
 #include "internal.h"
 
 namespace opsblas {
 
-constexpr int kCgBM = 64, kCgBN = 64, kCgBK = 8, kCgThreads = 256;
+constexpr int kCgBM = 64, kCgBN = 64, kCgBK = 8, kCgThreads = 128;
 
 // Element (r, c) of op(X) for op code OP (0 = N, 1 = T, 2 = C): X(r, c), X(c, r), conj(X(c, r)).
 template <int OP>
@@ -31,30 +32,40 @@ __device__ __forceinline__ float2 cg_load_op(const float2* X, int ld, int r, int
     return v;
 }
 
+// The four sums of a thread's 8 x 4 complex outputs (rows 4 tx .. and 32 + 4 tx .., columns 4 ty ..), rows
+// in packed pairs. A step loads 24 floats a thread for 128 fmas: shared memory returns 128 bytes a clock
+// to the registers of an SM, broadcast or not, so a 4 x 4 block (16 floats for 64) needs the whole of
+// it at the FMA rate. us, 4 x 4 scalar blocks with 8-byte C accesses -> these: 64^3 x 16384 1028 -> 912,
+// T 70 x 50 x 90 x 2048 339 -> 287, 128^3 x 1024 596 -> 600 (8 warps an SM instead of 16).
 struct CgAcc {
-    float t1[4][4], t2[4][4], t3[4][4], t4[4][4];
+    f32x2 t1[4][4], t2[4][4], t3[4][4], t4[4][4];
 };
 
-// One k step of the 4 x 4 complex outputs of thread (tx, ty).
 __device__ __forceinline__ void cg_step(const float (*Ar)[kCgBM + 4], const float (*Ai)[kCgBM + 4],
                                         const float (*Br)[kCgBN + 4], const float (*Bi)[kCgBN + 4], int kk, int tx,
                                         int ty, CgAcc& s)
 {
-    const float4 ar4 = *reinterpret_cast<const float4*>(&Ar[kk][tx * 4]);
-    const float4 ai4 = *reinterpret_cast<const float4*>(&Ai[kk][tx * 4]);
+    f32x2 ar[4], ai[4];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const ulonglong2 r = *reinterpret_cast<const ulonglong2*>(&Ar[kk][tx * 4 + 32 * h]);
+        const ulonglong2 i = *reinterpret_cast<const ulonglong2*>(&Ai[kk][tx * 4 + 32 * h]);
+        ar[2 * h] = r.x, ar[2 * h + 1] = r.y, ai[2 * h] = i.x, ai[2 * h + 1] = i.y;
+    }
     const float4 br4 = *reinterpret_cast<const float4*>(&Br[kk][ty * 4]);
     const float4 bi4 = *reinterpret_cast<const float4*>(&Bi[kk][ty * 4]);
-    const float ar[4] = {ar4.x, ar4.y, ar4.z, ar4.w}, ai[4] = {ai4.x, ai4.y, ai4.z, ai4.w};
-    const float br[4] = {br4.x, br4.y, br4.z, br4.w}, bi[4] = {bi4.x, bi4.y, bi4.z, bi4.w};
+    const float brv[4] = {br4.x, br4.y, br4.z, br4.w}, biv[4] = {bi4.x, bi4.y, bi4.z, bi4.w};
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int j = 0; j < 4; j++) {
+        const f32x2 br = f2_dup(brv[j]), bi = f2_dup(biv[j]);
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            s.t1[i][j] = fmaf(ar[i], br[j], s.t1[i][j]);
-            s.t2[i][j] = fmaf(ai[i], bi[j], s.t2[i][j]);
-            s.t3[i][j] = fmaf(ar[i], bi[j], s.t3[i][j]);
-            s.t4[i][j] = fmaf(ai[i], br[j], s.t4[i][j]);
+        for (int i = 0; i < 4; i++) {
+            s.t1[i][j] = f2_fma(ar[i], br, s.t1[i][j]);
+            s.t2[i][j] = f2_fma(ai[i], bi, s.t2[i][j]);
+            s.t3[i][j] = f2_fma(ar[i], bi, s.t3[i][j]);
+            s.t4[i][j] = f2_fma(ai[i], br, s.t4[i][j]);
         }
+    }
 }
 
 constexpr int kCgLoads = kCgBM * kCgBK / kCgThreads;  // elements per thread and operand slice
@@ -118,12 +129,12 @@ cgemm_batched_kernel(int m, int n, int k, float2 alpha, float2 beta, const float
     float2* C = Carray[b];
     if (C == nullptr) return;  // the whole CTA leaves before its first barrier
     const int m0 = (int)(blockIdx.x % tiles_m) * kCgBM, n0 = blockIdx.y * kCgBN;
-    const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+    const int tid = threadIdx.x, tx = tid % 8, ty = tid / 8;
     CgAcc s;
 #pragma unroll
     for (int i = 0; i < 4; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) s.t1[i][j] = s.t2[i][j] = s.t3[i][j] = s.t4[i][j] = 0.0f;
+        for (int j = 0; j < 4; j++) s.t1[i][j] = s.t2[i][j] = s.t3[i][j] = s.t4[i][j] = 0ull;
 
     if (k > 0) {
         const float2* A = Aarray[b];
@@ -155,27 +166,56 @@ cgemm_batched_kernel(int m, int n, int k, float2 alpha, float2 beta, const float
     }
 
     const bool has_beta = beta.x != 0.0f || beta.y != 0.0f;
+    auto combine = [&](int i, int j, float2 c) {
+        const float pr = __fsub_rn(f2_get(s.t1[i / 2][j], i & 1), f2_get(s.t2[i / 2][j], i & 1));
+        const float pi = __fadd_rn(f2_get(s.t3[i / 2][j], i & 1), f2_get(s.t4[i / 2][j], i & 1));
+        float cr = __fsub_rn(__fmul_rn(pr, alpha.x), __fmul_rn(pi, alpha.y));
+        float ci = __fadd_rn(__fmul_rn(pi, alpha.x), __fmul_rn(pr, alpha.y));
+        if (has_beta) {
+            cr = __fadd_rn(cr, __fmul_rn(c.x, beta.x));
+            ci = __fadd_rn(ci, __fmul_rn(c.y, beta.x));
+            cr = __fsub_rn(cr, __fmul_rn(c.y, beta.y));
+            ci = __fadd_rn(ci, __fmul_rn(c.x, beta.y));
+        }
+        return make_float2(cr, ci);
+    };
+    // Four rows of a column are one 32-byte sector: two 16-byte accesses where C is aligned for them (one
+    // 8-byte access a row touched every sector four times).
+    const bool aligned = (ldc & 1) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int gi = m0 + tx * 4 + i;
-        if (gi >= m) continue;
+    for (int h = 0; h < 2; h++) {
+        const int g0 = m0 + tx * 4 + 32 * h;
+        if (g0 >= m) break;
+        const bool vec = aligned && g0 + 3 < m;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const int gj = n0 + ty * 4 + j;
-            if (gj >= n) continue;
-            const long long idx = gi + (long long)gj * ldc;
-            const float pr = __fsub_rn(s.t1[i][j], s.t2[i][j]);
-            const float pi = __fadd_rn(s.t3[i][j], s.t4[i][j]);
-            float cr = __fsub_rn(__fmul_rn(pr, alpha.x), __fmul_rn(pi, alpha.y));
-            float ci = __fadd_rn(__fmul_rn(pi, alpha.x), __fmul_rn(pr, alpha.y));
+            if (gj >= n) break;
+            float2* c = C + g0 + (long long)gj * ldc;
+            float2 v[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) v[i] = make_float2(0.0f, 0.0f);
             if (has_beta) {
-                const float2 c = C[idx];
-                cr = __fadd_rn(cr, __fmul_rn(c.x, beta.x));
-                ci = __fadd_rn(ci, __fmul_rn(c.y, beta.x));
-                cr = __fsub_rn(cr, __fmul_rn(c.y, beta.y));
-                ci = __fadd_rn(ci, __fmul_rn(c.x, beta.y));
+                if (vec) {
+                    const float4 x = reinterpret_cast<const float4*>(c)[0], y = reinterpret_cast<const float4*>(c)[1];
+                    v[0] = make_float2(x.x, x.y), v[1] = make_float2(x.z, x.w);
+                    v[2] = make_float2(y.x, y.y), v[3] = make_float2(y.z, y.w);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; i++)
+                        if (g0 + i < m) v[i] = c[i];
+                }
             }
-            C[idx] = make_float2(cr, ci);
+#pragma unroll
+            for (int i = 0; i < 4; i++) v[i] = combine(4 * h + i, j, v[i]);
+            if (vec) {
+                reinterpret_cast<float4*>(c)[0] = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
+                reinterpret_cast<float4*>(c)[1] = make_float4(v[2].x, v[2].y, v[3].x, v[3].y);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+                    if (g0 + i < m) c[i] = v[i];
+            }
         }
     }
 }
