@@ -30,7 +30,9 @@
 //   matrix stops (info = column + 1); its later updates change nothing.
 #include <cuda_runtime.h>
 
+#include "f32x2.cuh"
 #include "internal.h"
+#include "lu_mid.cuh"
 #include "small_common.cuh"
 #include "tc_common.cuh"
 
@@ -38,13 +40,17 @@ namespace opsblas {
 
 constexpr int kBpW = 32;  // panel width = the update's K
 
+constexpr int kBpH = 16;  // columns factored at a time: half a panel, so that its unrolled code is run twice
+
+template <int NW>
 struct __align__(16) BpSmem {
-    float crow[2][32][kBpW];  // per column parity and warp: the warp's pivot candidate row
-    // per column (mod 3) the CTA's best pivot candidate: key << 5 | warp, by atomicMax; the
-    // exact search keys on the magnitude bits and then the position, the mixed one on its
-    // 32-bit approximate key
-    unsigned long long pkey[3];
-    float l11[kBpW][kBpW + 1];
+    union {
+        float crow[kBpH][NW][kBpH];  // per column and warp: the warp's pivot candidate row
+        float l11[kBpW][kBpW];       // after the factorisation: L11 negated
+    };
+    uint2 slot[2][NW];           // per column parity and warp: its best magnitude (bits) and position
+    int win[kBpH];               // the warp whose candidate became column c's pivot row
+    float u[kBpH][kBpH + 4];     // the first half's pivot rows, second half
     int mv_src[2 * kBpW];     // rows whose position changed: memory row and destination row
     int mv_dst[2 * kBpW];
     int mv_cnt;
@@ -187,18 +193,154 @@ lu_rows_out_kernel(float* const* __restrict__ LUarr, int ld, int n)
 // for the small CTAs, so that their shared memory lets more of them share an SM).
 template <int NT>
 struct PanelMv {
-    static constexpr int MVC = NT >= 128 ? 64 : 32;  // two buffers of 64 x MVC floats
+    static constexpr int MVC = NT == 128 || NT == 256 ? 64 : 32;  // two buffers of 64 x MVC floats
 };
 
+__device__ __forceinline__ void bp_take_row(f32x2 (&p)[kBpH / 2], const float* s)
+{
+#pragma unroll
+    for (int q = 0; q < kBpH / 4; q++) {
+        const ulonglong2 v = reinterpret_cast<const ulonglong2*>(s)[q];
+        p[2 * q] = v.x;
+        p[2 * q + 1] = v.y;
+    }
+}
+
+// Factors hw columns (k .. of half h) of the panel held in p: one CTA barrier per column. Each warp finds
+// its first maximum (two redux), publishes magnitude, position and the row; after the barrier every
+// warp takes the best of the warps' (two redux) and reads the pivot row. Returns the columns eliminated.
+// Multipliers are correctly rounded quotients by one reciprocal, and a row that has become a pivot is
+// poisoned with NaN until the half is done (both as in lu_mid.cuh: masks cost more than the updates).
+template <int NT, int RPT, bool PIVOT>
+__device__ __forceinline__ int lu_panel_half(f32x2 (&p)[RPT][kBpH / 2], int (&pos)[RPT], BpSmem<NT / 32>& S, int k,
+                                             int hw, int* __restrict__ piv, int tid, int warp, int lane)
+{
+    constexpr int NW = NT / 32;
+    constexpr float lo = 0x1p-60f, hi = 0x1p60f;
+    int done = hw;
+#pragma unroll
+    for (int c = 0; c < kBpH; c++, k++) {
+        if (c >= hw) break;
+        float a[RPT];
+#pragma unroll
+        for (int r = 0; r < RPT; r++) a[r] = f2_get(p[r][c / 2], c & 1);
+        int ppos = k, bw = 0;
+        bool usual = false;
+        float y = 0.0f;
+        if (PIVOT) {
+            float best = fabsf(a[0]);
+#pragma unroll
+            for (int r = 1; r < RPT; r++) best = fmaxf(best, fabsf(a[r]));
+            const float wm = warp_absmax(best);  // (NaN, the dead rows' value, never wins)
+            unsigned cand = 0x7fffffffu;
+#pragma unroll
+            for (int r = 0; r < RPT; r++)
+                if (fabsf(a[r]) == wm) cand = min(cand, (unsigned)pos[r]);
+            if (!(wm > 0.0f)) {  // nothing above zero: the warp's lowest live position (warp-uniform)
+#pragma unroll
+                for (int r = 0; r < RPT; r++)
+                    if (pos[r] >= k) cand = min(cand, (unsigned)pos[r]);
+            }
+            const int wp = (int)__reduce_min_sync(0xffffffffu, cand);
+            if (lane == 0) S.slot[c & 1][warp] = make_uint2(wm > 0.0f ? __float_as_uint(wm) : 0u, (unsigned)wp);
+#pragma unroll
+            for (int r = 0; r < RPT; r++)
+                if (pos[r] == wp) {
+                    ulonglong2* d = reinterpret_cast<ulonglong2*>(S.crow[c][warp]);
+#pragma unroll
+                    for (int q = 0; q < kBpH / 4; q++) d[q] = make_ulonglong2(p[r][2 * q], p[r][2 * q + 1]);
+                }
+            __syncthreads();
+            const uint2 sl = lane < NW ? S.slot[c & 1][lane] : make_uint2(0u, 0x7fffffffu);
+            const unsigned g = __reduce_max_sync(0xffffffffu, sl.x);
+            ppos = (int)__reduce_min_sync(0xffffffffu, sl.x == g ? sl.y : 0x7fffffffu);
+            bw = __ffs(__ballot_sync(0xffffffffu, sl.y == (unsigned)ppos)) - 1;
+            const float mx = __uint_as_float(g);
+            y = mid_reciprocal(mx);
+            usual = mx >= lo && mx <= hi;
+        } else {  // the row at position k, published by its warp
+#pragma unroll
+            for (int r = 0; r < RPT; r++)
+                if (pos[r] == k) {
+                    S.win[c] = warp;
+                    ulonglong2* d = reinterpret_cast<ulonglong2*>(S.crow[c][warp]);
+#pragma unroll
+                    for (int q = 0; q < kBpH / 4; q++) d[q] = make_ulonglong2(p[r][2 * q], p[r][2 * q + 1]);
+                }
+            __syncthreads();
+            bw = S.win[c];
+        }
+        const float* prow = S.crow[c][bw];
+        f32x2 u[kBpH / 2];
+#pragma unroll
+        for (int q = c / 4; q < kBpH / 4; q++) {
+            const ulonglong2 v = reinterpret_cast<const ulonglong2*>(prow)[q];
+            u[2 * q] = v.x;
+            u[2 * q + 1] = v.y;
+        }
+        const float pv = f2_get(u[c / 2], c & 1);
+        if (tid == 0) {
+            if (PIVOT) {
+                piv[k] = ppos + 1;
+                S.win[c] = bw;
+            }
+        }
+        if (!usual && pv == 0.0f) {  // exactly-zero pivot: stop here, before the interchange (uniform)
+            done = c;
+            break;
+        }
+        y = copysignf(y, pv);
+        float l[RPT];
+        float least = fabsf(a[0]);
+#pragma unroll
+        for (int r = 0; r < RPT; r++) {
+            if (r > 0) least = fminf(least, fabsf(a[r]));
+            l[r] = __fmul_rn(a[r], y);
+            l[r] = fmaf(fmaf(-l[r], pv, a[r]), y, l[r]);
+            l[r] = fmaf(fmaf(-l[r], pv, a[r]), y, l[r]);
+        }
+        if (!usual || least < lo) {
+#pragma unroll
+            for (int r = 0; r < RPT; r++)
+                if (!usual || fabsf(a[r]) < lo) l[r] = a[r] / pv;
+        }
+#pragma unroll
+        for (int r = 0; r < RPT; r++) {
+            const bool hit = pos[r] == ppos;
+            if (pos[r] == k) pos[r] = ppos;
+            if (hit) pos[r] = k;
+            const float v = hit ? __int_as_float(0x7fffffff) : -l[r];
+            float x, z;
+            f2_unpack(p[r][c / 2], x, z);
+            if (c & 1)
+                p[r][c / 2] = f2_pack(x, l[r]);
+            else
+                p[r][c / 2] = f2_pack(l[r], fmaf(f2_get(u[c / 2], 1), v, z));
+            const f32x2 nl = f2_dup(v);
+#pragma unroll
+            for (int h = c / 2 + 1; h < kBpH / 2; h++) p[r][h] = f2_fma(u[h], nl, p[r][h]);
+        }
+    }
+    // the half's pivot rows, overwritten after they were published
+#pragma unroll
+    for (int r = 0; r < RPT; r++) {
+        const int i = pos[r] - (k - done);
+        if (pos[r] >= k - done && pos[r] < k) bp_take_row(p[r], S.crow[i][warp]);
+    }
+    return done;
+}
+
 // One CTA per matrix; thread t holds memory rows k0 + t + r * NT (r < RPT) of the panel. NT x RPT
-// covers the panel's rows; 128 registers a thread, so that 512 / NT CTAs share an SM.
-// EXACT (the plain FP32 factorisation): the reference's arithmetic -- first maximum of the exact
-// magnitudes, true division, and after a stop at column kk of the panel only the U rows above kk
-// (the trailing update then takes rows from kk on with K = kk - k0); no TF32 planes (the update
-// reads L21 and U12 from LU). Otherwise (mixed): the approximate pivot key and reciprocal, TF32
-// planes, and a stop zeroes the update. PIVOT = false: no pivoting (the reference's no-pivot
-// variant). st[m]: the matrix's info code so far (0, or the stop column + 1); info, when not
-// nullptr, receives the same.
+// covers the panel's rows; 128 registers a thread, so that 512 / NT CTAs share an SM. The panel is
+// factored in two halves of 16 columns by the same code (a whole panel's unrolled columns are more code
+// than the instruction cache holds: half of the former kernel's time was waiting for instructions).
+// The pivot search is the reference's first maximum of the exact magnitudes, the multipliers are
+// correctly rounded, every update one fmaf in column order.
+// EXACT (the plain FP32 factorisation): after a stop at column kk of the panel only the U rows above kk
+// are formed (the trailing update then takes rows from kk on with K = kk - k0); no TF32 planes (the
+// update reads L21 and U12 from LU). Otherwise (mixed): TF32 planes, and a stop zeroes the update.
+// PIVOT = false: no pivoting (the reference's no-pivot variant). st[m]: the matrix's info code so far
+// (0, or the stop column + 1); info, when not nullptr, receives the same.
 template <int NT, int RPT, bool EXACT, bool PIVOT>
 __global__ void __launch_bounds__(NT, 512 / NT)
 lu_panel_kernel(float* const* __restrict__ LUarr, int n, int ldt, int k0, int* __restrict__ piv,
@@ -206,7 +348,7 @@ lu_panel_kernel(float* const* __restrict__ LUarr, int n, int ldt, int k0, int* _
                 long long u12_off, long long per_matrix)
 {
     constexpr int NW = NT / 32;
-    __shared__ BpSmem S;
+    __shared__ BpSmem<NW> S;
     constexpr int kMvCols = PanelMv<NT>::MVC;
     __shared__ __align__(16) float mvbuf[2][2 * kBpW * kMvCols];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -223,11 +365,7 @@ lu_panel_kernel(float* const* __restrict__ LUarr, int n, int ldt, int k0, int* _
     // whole rows as float4 when every row start is 16-byte aligned (uniform per matrix)
     const bool vec = (reinterpret_cast<uintptr_t>(T) & 15) == 0 && (ldt & 3) == 0 && pw == kBpW;
 
-    if (tid == 0) {
-        S.mv_cnt = 0;
-        S.pkey[0] = 0ull;
-        S.pkey[1] = 0ull;
-    }
+    if (tid == 0) S.mv_cnt = 0;
     if (inf0 != 0) {  // stopped at an earlier zero pivot
         if (!EXACT) {  // this step's update must change nothing
             for (int e = tid; e < (ntr > 0 ? ntr : 0) * kBpW; e += NT) {
@@ -240,191 +378,139 @@ lu_panel_kernel(float* const* __restrict__ LUarr, int n, int ldt, int k0, int* _
         return;
     }
 
-    // 1. this thread's panel rows (zeros outside the matrix)
-    bool valid[RPT];
+    // 1. this thread's panel rows (zeros outside the matrix; no position: -1): cur is the half being
+    //    factored, oth the other one
     int pos[RPT];
-    float p[RPT][kBpW];
+    f32x2 cur[RPT][kBpH / 2], oth[RPT][kBpH / 2];
 #pragma unroll
     for (int r = 0; r < RPT; r++) {
-        valid[r] = tid + r * NT < mp;
-        pos[r] = k0 + tid + r * NT;
+        const bool valid = tid + r * NT < mp;
+        pos[r] = valid ? k0 + tid + r * NT : -1;
 #pragma unroll
-        for (int c = 0; c < kBpW; c++) p[r][c] = 0.0f;
-        if (valid[r]) {
+        for (int h = 0; h < kBpH / 2; h++) cur[r][h] = oth[r][h] = f2_dup(__int_as_float(0x7fffffff));
+        if (valid) {
             const float* row = T + (long long)pos[r] * ldt + k0;
             if (vec) {
 #pragma unroll
-                for (int q = 0; q < kBpW / 4; q++) {
-                    const float4 v = reinterpret_cast<const float4*>(row)[q];
-                    p[r][4 * q] = v.x;
-                    p[r][4 * q + 1] = v.y;
-                    p[r][4 * q + 2] = v.z;
-                    p[r][4 * q + 3] = v.w;
+                for (int q = 0; q < kBpH / 4; q++) {
+                    const ulonglong2 v = reinterpret_cast<const ulonglong2*>(row)[q];
+                    const ulonglong2 x = reinterpret_cast<const ulonglong2*>(row + kBpH)[q];
+                    cur[r][2 * q] = v.x, cur[r][2 * q + 1] = v.y;
+                    oth[r][2 * q] = x.x, oth[r][2 * q + 1] = x.y;
                 }
             } else {
 #pragma unroll
-                for (int c = 0; c < kBpW; c++)
-                    if (c < pw) p[r][c] = row[c];
+                for (int h = 0; h < kBpH / 2; h++) {
+                    const int c = 2 * h, e = kBpH + 2 * h;
+                    cur[r][h] = f2_pack(c < pw ? row[c] : 0.0f, c + 1 < pw ? row[c + 1] : 0.0f);
+                    oth[r][h] = f2_pack(e < pw ? row[e] : 0.0f, e + 1 < pw ? row[e + 1] : 0.0f);
+                }
             }
         }
     }
     __syncthreads();
 
-    // 2. factor, one CTA barrier per column
-    int done = pw;
+    // 2. factor, half by half; the second half first takes the first's update
+    int done = 0, first = 0;  // first: the columns eliminated in the first half
+#pragma unroll 1
+    for (int half = 0; half < 2; half++) {
+        const int hw = max(0, min(kBpH, pw - half * kBpH));
+        const int d = lu_panel_half<NT, RPT, PIVOT>(cur, pos, S, k0 + half * kBpH, hw, pm, tid, warp, lane);
+        done += d;
+        if (half == 1) break;
 #pragma unroll
-    for (int c = 0; c < kBpW; c++) {
-        if (c >= pw) break;
-        const int k = k0 + c;
-        const int buf = c & 1;
-        int ppos;
-        const float* prow;
-        bool nocand = false;  // (mixed search) no candidate key at all: treated as a zero pivot
-        if (!PIVOT) {  // the row at position k
+        for (int r = 0; r < RPT; r++)
+#pragma unroll
+            for (int h = 0; h < kBpH / 2; h++) {
+                const f32x2 x = cur[r][h];
+                cur[r][h] = oth[r][h];
+                oth[r][h] = x;
+            }
+        // the second half's entries of the first half's pivot rows, solved by a lane per column, then
+        // one fmaf per pivot row for the rows below (after a stop: the rows before it only)
+        if (pw > kBpH) {
 #pragma unroll
             for (int r = 0; r < RPT; r++)
-                if (valid[r] && pos[r] == k) {
-                    float4* dst = reinterpret_cast<float4*>(S.crow[buf][0]);
+                if (pos[r] >= k0 && pos[r] < k0 + d) {
+                    ulonglong2* x = reinterpret_cast<ulonglong2*>(S.u[pos[r] - k0]);
 #pragma unroll
-                    for (int q = 0; q < kBpW / 4; q++)
-                        dst[q] = make_float4(p[r][4 * q], p[r][4 * q + 1], p[r][4 * q + 2], p[r][4 * q + 3]);
+                    for (int q = 0; q < kBpH / 4; q++) x[q] = make_ulonglong2(cur[r][2 * q], cur[r][2 * q + 1]);
                 }
             __syncthreads();
-            ppos = k;
-            prow = S.crow[buf][0];
-        } else if (EXACT) {
-            // first maximum of |x| over the positions >= k: the largest magnitude (as its bits; NaN
-            // counts as zero and never wins), then the lowest position among equals
-            unsigned bm = 0u;
-            int bp = 0x7fffffff;
+            if (tid < kBpH) {
+                float x[kBpH];
 #pragma unroll
-            for (int r = 0; r < RPT; r++) {
-                if (!(valid[r] && pos[r] >= k)) continue;
-                const float av = fabsf(p[r][c]);
-                const unsigned mag = av == av ? __float_as_uint(av) : 0u;
-                if (mag > bm || (mag == bm && pos[r] < bp)) {
-                    bm = mag;
-                    bp = pos[r];
-                }
-            }
-            const unsigned wm = __reduce_max_sync(0xffffffffu, bm);
-            const int wp = (int)__reduce_min_sync(0xffffffffu, bm == wm ? (unsigned)bp : 0x7fffffffu);
-            // the warp's best into the CTA's: magnitude, then the lower position, then the warp
-            if (lane == 0 && wp != 0x7fffffff)
-                atomicMax(&S.pkey[c % 3], ((unsigned long long)wm << 32) |
-                                              ((unsigned long long)(1023 - (wp - k0)) << 5) | (unsigned)warp);
+                for (int i = 0; i < kBpH; i++) x[i] = i < d ? S.u[i][tid] : 0.0f;
 #pragma unroll
-            for (int r = 0; r < RPT; r++)
-                if (valid[r] && pos[r] == wp && bp == wp) {
-                    float4* dst = reinterpret_cast<float4*>(S.crow[buf][warp]);
+                for (int i = 1; i < kBpH; i++) {
+                    if (i < d) {
+                        const float* l = S.crow[i][S.win[i]];
 #pragma unroll
-                    for (int q = 0; q < kBpW / 4; q++)
-                        dst[q] = make_float4(p[r][4 * q], p[r][4 * q + 1], p[r][4 * q + 2], p[r][4 * q + 3]);
-                }
-            if (tid == 0) S.pkey[(c + 1) % 3] = 0ull;  // read last at column c - 2, before this barrier
-            __syncthreads();
-            const unsigned long long key = S.pkey[c % 3];  // (position k is always a candidate)
-            ppos = k0 + 1023 - (int)((key >> 5) & 1023u);
-            prow = S.crow[buf][(int)(key & 31u)];
-        } else {
-            unsigned best = 0u;  // this thread's best candidate key (0: none)
-#pragma unroll
-            for (int r = 0; r < RPT; r++) {
-                const float av = fabsf(p[r][c]);
-                const unsigned mag = (av == av) ? (__float_as_uint(av) >> 9) : 0u;  // NaN never wins
-                const unsigned key =
-                    (valid[r] && pos[r] >= k) ? ((mag << 10) | (1023u - (unsigned)(pos[r] - k0))) : 0u;
-                best = key > best ? key : best;
-            }
-            const unsigned wkey = __reduce_max_sync(0xffffffffu, best);
-            if (lane == 0 && wkey != 0u) atomicMax(&S.pkey[c % 3], ((unsigned long long)wkey << 5) | (unsigned)warp);
-            if (best != 0u && best == wkey) {  // keys are unique: one writer a warp
-                float4* dst = reinterpret_cast<float4*>(S.crow[buf][warp]);
-#pragma unroll
-                for (int r = 0; r < RPT; r++) {
-                    const float av = fabsf(p[r][c]);
-                    const unsigned mag = (av == av) ? (__float_as_uint(av) >> 9) : 0u;
-                    const unsigned key =
-                        (valid[r] && pos[r] >= k) ? ((mag << 10) | (1023u - (unsigned)(pos[r] - k0))) : 0u;
-                    if (key == best) {
-#pragma unroll
-                        for (int q = 0; q < kBpW / 4; q++)
-                            dst[q] = make_float4(p[r][4 * q], p[r][4 * q + 1], p[r][4 * q + 2], p[r][4 * q + 3]);
+                        for (int c = 0; c < kBpH; c++)
+                            if (c < i) x[i] = fmaf(-l[c], x[c], x[i]);
+                        S.u[i][tid] = x[i];
                     }
                 }
             }
-            if (tid == 0) S.pkey[(c + 1) % 3] = 0ull;  // read last at column c - 2, before this barrier
             __syncthreads();
-            const unsigned long long key = S.pkey[c % 3];
-            const unsigned bk = (unsigned)(key >> 5);
-            nocand = bk == 0u;
-            ppos = nocand ? k : k0 + 1023 - (int)(bk & 1023u);
-            prow = S.crow[buf][(int)(key & 31u)];
-        }
-        const float pv = prow[c];
-        if (PIVOT && tid == 0) pm[k] = ppos + 1;
-        if (pv == 0.0f || nocand) {  // exactly-zero pivot: stop here, before the interchange (uniform)
-            if (tid == 0) {
-                st[m] = k + 1;
-                if (info != nullptr && info != st) info[m] = k + 1;
-            }
-            done = c;
-            break;
-        }
-        float rinv = 0.0f;
-        if (!EXACT) asm("rcp.approx.f32 %0, %1;" : "=f"(rinv) : "f"(pv));
-        float l[RPT];
-        bool upd[RPT];  // rows below the pivot position take the update
 #pragma unroll
-        for (int r = 0; r < RPT; r++) {
-            if (PIVOT) {
-                if (pos[r] == ppos)
-                    pos[r] = k;
-                else if (pos[r] == k)
-                    pos[r] = ppos;
-            }
-            upd[r] = valid[r] && pos[r] > k;
-            l[r] = EXACT ? p[r][c] / pv : p[r][c] * rinv;
-            if (upd[r]) p[r][c] = l[r];
-        }
-        // p[j] -= l * u[j] for j > c: packed f32x2 fmas on the column pairs right of c (each lane
-        // an IEEE fma, fma(u, -l, p) == fmaf(-l, u, p) bit for bit)
+            for (int i = 0; i < kBpH; i++) {
+                if (i < d) {
+                    const ulonglong2* ui = reinterpret_cast<const ulonglong2*>(S.u[i]);
+                    f32x2 nl[RPT];
 #pragma unroll
-        for (int j = 0; j < kBpW; j += 2) {
-            if (j > c) {
-                const float2 u = make_float2(prow[j], prow[j + 1]);
+                    for (int r = 0; r < RPT; r++) nl[r] = f2_dup(-f2_get(oth[r][i / 2], i & 1));
 #pragma unroll
-                for (int r = 0; r < RPT; r++)
-                    if (upd[r]) {
-                        const float2 q = __ffma2_rn(u, make_float2(-l[r], -l[r]), make_float2(p[r][j], p[r][j + 1]));
-                        p[r][j] = q.x;
-                        p[r][j + 1] = q.y;
+                    for (int q = 0; q < kBpH / 4; q++) {
+                        const ulonglong2 v = ui[q];
+#pragma unroll
+                        for (int r = 0; r < RPT; r++) {
+                            cur[r][2 * q] = f2_fma(v.x, nl[r], cur[r][2 * q]);
+                            cur[r][2 * q + 1] = f2_fma(v.y, nl[r], cur[r][2 * q + 1]);
+                        }
                     }
-            } else if (j + 1 > c) {
-                const float u = prow[j + 1];
-#pragma unroll
-                for (int r = 0; r < RPT; r++)
-                    if (upd[r]) p[r][j + 1] = fmaf(-l[r], u, p[r][j + 1]);
+                }
             }
+#pragma unroll
+            for (int r = 0; r < RPT; r++)
+                if (pos[r] < k0 + d) {  // dead (their second half is in S.u), or no row
+#pragma unroll
+                    for (int h = 0; h < kBpH / 2; h++) cur[r][h] = f2_dup(__int_as_float(0x7fffffff));
+                }
         }
+        first = d;
+        if (d < hw) break;  // stopped in the first half
+    }
+    // (oth: columns 0..15, cur: 16..31) the second half of the first half's pivot rows
+    if (pw > kBpH) {
+#pragma unroll
+        for (int r = 0; r < RPT; r++)
+            if (pos[r] >= k0 && pos[r] < k0 + first) bp_take_row(cur[r], S.u[pos[r] - k0]);
     }
     const bool stopped = done < pw;
+    if (stopped && tid == 0) {
+        st[m] = k0 + done + 1;
+        if (info != nullptr && info != st) info[m] = k0 + done + 1;
+    }
+    __syncthreads();  // S.crow and S.u are read before l11 is used below; done is uniform
 
     // 3. the panel at its final rows; L21 (zero after a stop: the update then changes nothing) and
     //    L11; the rows whose position changed
+    auto elem = [&](int r, int c) { return f2_get(c < 16 ? oth[r][c % 16 / 2] : cur[r][c % 16 / 2], c & 1); };
 #pragma unroll
     for (int r = 0; r < RPT; r++) {
-        if (!valid[r]) continue;
+        if (pos[r] < 0) continue;
         float* row = T + (long long)pos[r] * ldt + k0;
         if (vec) {
 #pragma unroll
-            for (int q = 0; q < kBpW / 4; q++)
-                reinterpret_cast<float4*>(row)[q] =
-                    make_float4(p[r][4 * q], p[r][4 * q + 1], p[r][4 * q + 2], p[r][4 * q + 3]);
+            for (int q = 0; q < kBpH / 4; q++) {
+                reinterpret_cast<ulonglong2*>(row)[q] = make_ulonglong2(oth[r][2 * q], oth[r][2 * q + 1]);
+                reinterpret_cast<ulonglong2*>(row + kBpH)[q] = make_ulonglong2(cur[r][2 * q], cur[r][2 * q + 1]);
+            }
         } else {
 #pragma unroll
             for (int c = 0; c < kBpW; c++)
-                if (c < pw) row[c] = p[r][c];
+                if (c < pw) row[c] = elem(r, c);
         }
         if (PIVOT && pos[r] != k0 + tid + r * NT) {
             const int q = atomicAdd(&S.mv_cnt, 1);
@@ -438,14 +524,14 @@ lu_panel_kernel(float* const* __restrict__ LUarr, int n, int ldt, int k0, int* _
             for (int q = 0; q < kBpW / 4; q++) {
                 float h[4], lw[4];
 #pragma unroll
-                for (int e = 0; e < 4; e++) tf32_split(stopped ? 0.0f : p[r][4 * q + e], h[e], lw[e]);
+                for (int e = 0; e < 4; e++) tf32_split(stopped ? 0.0f : elem(r, 4 * q + e), h[e], lw[e]);
                 dh[q] = make_float4(h[0], h[1], h[2], h[3]);
                 dl[q] = make_float4(lw[0], lw[1], lw[2], lw[3]);
             }
         }
         if (pos[r] < k0 + kBpW) {
 #pragma unroll
-            for (int c = 0; c < kBpW; c++) S.l11[pos[r] - k0][c] = p[r][c];
+            for (int c = 0; c < kBpW; c++) S.l11[pos[r] - k0][c] = -elem(r, c);
         }
     }
     __syncthreads();
@@ -509,22 +595,39 @@ lu_panel_kernel(float* const* __restrict__ LUarr, int n, int ldt, int k0, int* _
     // 5. U12 = L11^-1 * (the pivot rows' trailing entries, now in rows k0..k0+31), one thread per
     //    trailing column, in the reference's order (row i takes columns 0..i-1 in turn): the final U
     //    rows (above the stop column only, EXACT) and the TF32 planes of the update (mixed)
-    const int urows = EXACT ? done : kBpW;
+    if (stopped) {
+        for (int jj = tid; jj < ntr; jj += NT) {
+            if (EXACT) {  // rows above the stop, one at a time
+                float* t = T + (long long)k0 * ldt + k0 + kBpW + jj;
+                for (int i = 1; i < done; i++) {
+                    float x = t[(long long)i * ldt];
+                    for (int c = 0; c < i; c++) x = fmaf(S.l11[i][c], t[(long long)c * ldt], x);
+                    t[(long long)i * ldt] = x;
+                }
+            } else {
+                for (int q = 0; q < kBpW; q++) U12[(long long)jj * kBpW + q] = U12[lo + (long long)jj * kBpW + q] = 0.0f;
+            }
+        }
+        return;
+    }
     for (int jj = tid; jj < ntr; jj += NT) {
-        const int col = k0 + kBpW + jj;
+        float* t = T + (long long)k0 * ldt + k0 + kBpW + jj;
         float u[kBpW];
 #pragma unroll
-        for (int i = 0; i < kBpW; i++) u[i] = (stopped && !EXACT) ? 0.0f : T[(long long)(k0 + i) * ldt + col];
+        for (int i = 0; i < kBpW; i++) u[i] = t[(long long)i * ldt];
 #pragma unroll
-        for (int i = 1; i < kBpW; i++)
+        for (int i = 1; i < kBpW; i++) {
 #pragma unroll
-            for (int c = 0; c < kBpW; c++)
-                if (c < i && i < urows) u[i] = fmaf(-S.l11[i][c], u[c], u[i]);
-        if (EXACT || !stopped) {
+            for (int q = 0; q < (i + 3) / 4; q++) {
+                const float4 v = reinterpret_cast<const float4*>(S.l11[i])[q];
+                const float l[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-            for (int i = 1; i < kBpW; i++)
-                if (i < urows) T[(long long)(k0 + i) * ldt + col] = u[i];
+                for (int e = 0; e < 4; e++)
+                    if (4 * q + e < i) u[i] = fmaf(l[e], u[4 * q + e], u[i]);
+            }
         }
+#pragma unroll
+        for (int i = 1; i < kBpW; i++) t[(long long)i * ldt] = u[i];
         if (!EXACT) {
             float4* dh = reinterpret_cast<float4*>(U12 + (long long)jj * kBpW);
             float4* dl = reinterpret_cast<float4*>(U12 + lo + (long long)jj * kBpW);
