@@ -73,6 +73,10 @@ inline int max1(int n) { return n > 1 ? n : 1; }
 // pass NULL for converged matrices).
 cudaError_t getrs_launch(cudaStream_t st, bool trans, int n, int nrhs, const float* const* Aarray, int lda,
                          const int* devIpiv, float* const* Barray, int ldb, int batchCount);
+// getrs_block.cu: trans N, 128 < n <= 256, right-hand sides in registers.
+bool getrs_block_preferred(int n, int nrhs, int batch);
+cudaError_t getrs_block_launch(cudaStream_t st, int n, int nrhs, const float* const* Aarray, int lda, const int* ipiv,
+                               float* const* Barray, int ldb, int batch);
 // getrs_blk.cu: trans N, n > 128, blocked substitution with the right-hand sides in shared memory.
 bool getrs_blk_supported(int n);
 cudaError_t getrs_blk_launch(cudaStream_t st, int n, int nrhs, const float* const* Aarray, int lda, const int* ipiv,

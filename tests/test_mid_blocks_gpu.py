@@ -114,3 +114,29 @@ def test_getrs_staged_edges(handle, n, trans):
         B = to_dev(b, "cuda")
         handle.getrs(trans, to_dev(lu, "cuda"), n, ld, to_dev(piv, "cuda"), B, nrhs, ld)
         assert_bitwise(to_host(B), want, f"n={n} nrhs={nrhs} {trans}")
+
+
+@pytest.mark.parametrize("n", [129, 144, 160, 161, 191, 192, 193, 224, 255, 256])
+def test_getrs_block_edges(handle, n):
+    """The register solve (getrs_block.cu): panel and tile edges, column counts around 4, 16 and a CTA's 64, odd
+    strides, invalid pivots, a zero on the diagonal, infinities and NaN."""
+    rng = np.random.default_rng(n)
+    for nrhs, batch, pad in ((1, 300, 0), (4, 300, 1), (5, 300, 4), (16, 3, 0), (17, 160, 0), (70, 60, 3)):
+        ld = n + pad
+        lu = rng.standard_normal((batch, n, ld)).astype(np.float32)
+        lu[:, np.arange(n), np.arange(n)] += 12
+        piv = (np.arange(1, n + 1) + rng.integers(0, n - np.arange(n), (batch, n))).astype(np.int32)
+        piv[0, 0] = 0
+        piv[0, n - 1] = n + 7
+        if batch > 1:
+            lu[1, n // 2, n // 2] = 0.0
+        b = rng.standard_normal((batch, nrhs, ld)).astype(np.float32)
+        if nrhs > 2:
+            b[batch - 1, 1, n - 1] = np.inf
+            b[batch - 1, 2, 0] = np.nan
+        want = b.copy()
+        with np.errstate(all="ignore"):
+            O.port_getrs("N", lu, n, ld, piv, want, nrhs, ld)
+        B = to_dev(b, "cuda")
+        handle.getrs("N", to_dev(lu, "cuda"), n, ld, to_dev(piv, "cuda"), B, nrhs, ld)
+        assert_bitwise(to_host(B), want, f"n={n} nrhs={nrhs}")
