@@ -86,16 +86,27 @@ __device__ __forceinline__ void grouped_mid(const GroupDev& g, int li, float* co
 }
 
 // Classes of orders and how the CTA's twelve warps and its shared memory are dealt out to each: as many
-// matrices at a time as the memory holds, 4 warps each above 96 rows, 2 above 64, 1 below.
-constexpr int kGrpClasses = 5;  // 97..128, 81..96, 65..80, 33..64, 1..32
-__host__ __device__ constexpr int grp_class(int n) { return n > 96 ? 0 : n > 80 ? 1 : n > 64 ? 2 : n > 32 ? 3 : 4; }
+// matrices at a time as the memory (or the sixteen barriers) hold, with the warps a matrix that were
+// fastest in the batched kernel at that number of matrices an SM (getrf_mid.cu).
+constexpr int kGrpClasses = 6;  // 113..128, 97..112, 81..96, 65..80, 33..64, 1..32
+__host__ __device__ constexpr int grp_class(int n)
+{
+    return n > 112 ? 0 : n > 96 ? 1 : n > 80 ? 2 : n > 64 ? 3 : n > 32 ? 4 : 5;
+}
 __host__ __device__ constexpr int grp_team_warps(int c) { return c == 0 ? 4 : c < 3 ? 2 : 1; }
-__host__ __device__ constexpr int grp_teams(int c) { return c == 0 ? 3 : c < 3 ? 5 : c == 3 ? 11 : 12; }
+__host__ __device__ constexpr int grp_teams(int c)
+{
+    return c == 0 ? 3 : c == 1 ? 4 : c == 2 ? 5 : c == 3 ? 7 : c == 4 ? 11 : 12;
+}
 __host__ __device__ constexpr size_t grp_region(int c)
 {
-    return c == 0 ? sizeof(MidSmem<8, 4>) : c == 1 ? sizeof(MidSmem<6, 2>) : c == 2 ? sizeof(MidSmem<5, 2>)
-           : c == 3 ? sizeof(MidSmem<4, 1>) : 3 * 32 * sizeof(float);  // small: two row buffers, owners
+    return c == 0 ? sizeof(MidSmem<8, 4>) : c == 1 ? sizeof(MidSmem<7, 2>) : c == 2 ? sizeof(MidSmem<6, 2>)
+           : c == 3 ? sizeof(MidSmem<5, 1>) : c == 4 ? sizeof(MidSmem<4, 1>)
+                                            : 3 * 32 * sizeof(float);  // small: two row buffers, owners
 }
+static_assert(grp_teams(0) * grp_region(0) <= 231000 && grp_teams(1) * grp_region(1) <= 231000 &&
+              grp_teams(2) * grp_region(2) <= 231000 && grp_teams(3) * grp_region(3) <= 231000 &&
+              grp_teams(4) * grp_region(4) <= 231000, "one CTA an SM");
 
 // ----------------------------------------------------------------------------- n <= 32 --
 template <int N, int SEG>
@@ -177,16 +188,9 @@ __device__ __forceinline__ void grouped_class(const GroupDev* groups, const Grou
         if (t >= count) break;
         const GroupTask task = tasks[t];
         const GroupDev& g = groups[task.group];  // fields read when needed: fewer live registers
-        if constexpr (C == 0) {
-            if (g.n > 112)
-                grouped_mid<8, W>(g, task.first, Aarray, Barray, piv, info, region, warp, lane, bar);
-            else
-                grouped_mid<7, W>(g, task.first, Aarray, Barray, piv, info, region, warp, lane, bar);
-        } else if constexpr (C == 1) {
-            grouped_mid<6, W>(g, task.first, Aarray, Barray, piv, info, region, warp, lane, bar);
-        } else if constexpr (C == 2) {
-            grouped_mid<5, W>(g, task.first, Aarray, Barray, piv, info, region, warp, lane, bar);
-        } else if constexpr (C == 3) {
+        if constexpr (C < 4) {
+            grouped_mid<8 - C, W>(g, task.first, Aarray, Barray, piv, info, region, warp, lane, bar);
+        } else if constexpr (C == 4) {
             if (g.n > 48)
                 grouped_mid<4, W>(g, task.first, Aarray, Barray, piv, info, region, warp, lane, bar);
             else
@@ -233,6 +237,7 @@ grouped_lu_kernel(const GroupDev* groups, const GroupTask* __restrict__ tasks, c
     OPSBLAS_GROUPED_CLASS(2)
     OPSBLAS_GROUPED_CLASS(3)
     OPSBLAS_GROUPED_CLASS(4)
+    OPSBLAS_GROUPED_CLASS(5)
 #undef OPSBLAS_GROUPED_CLASS
 
     // the last CTA out resets the counters for the next execution
