@@ -229,3 +229,13 @@ def test_grouped_tuning_table_is_read(ob, handle, tmp_path, monkeypatch):
     plan = ob.GroupedPlan(handle, [8, 40, 100], [1, 1, 1], [2, 2, 2])
     assert plan.config() == [(32, 0, 0), (0, 4, 3), (0, 8, 4)]
     plan.close()
+
+
+def test_grouped_class_edges(ob, handle):
+    """Orders on both sides of every class of the persistent kernel, from fewer matrices than teams to several
+    rounds of them, with padding, singular members and several right-hand sides."""
+    ns = [1, 32, 33, 64, 65, 80, 81, 96, 97, 112, 113, 128]
+    for seed, (size, pad, nrhs) in enumerate([(1, 0, 1), (37, 3, 5), (700, 0, 1)]):
+        d = _setup(ob, ns, [nrhs] * len(ns), [size] * len(ns), 40 + seed, ldpad=pad, singular=(2, 30, 100, 301))
+        outs, ref, _ = _run_both(ob, handle, d)
+        _assert_same(outs[0], ref)
