@@ -4,6 +4,7 @@
 // LU crosses HBM once. Bit-identical to the reference's order (sgetrs_batched_kernel.cpp:83-200).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "internal.h"
@@ -17,7 +18,7 @@ constexpr int kGbMaxWarps = 4;
 template <int R, int CW>
 __global__ void __launch_bounds__(kGbMaxWarps * 32, CW > 8 && R > 6 ? 2 : 4)
 getrs_block_kernel(const float* const* __restrict__ Aarray, int n, int lda, const int* __restrict__ ipiv,
-                   float* const* __restrict__ Barray, int ldb, int nrhs)
+                   float* const* __restrict__ Barray, int ldb, int nrhs, int first)
 {
     constexpr int LDP = 32 * R + 4;
     extern __shared__ __align__(16) float sm[];
@@ -50,8 +51,9 @@ getrs_block_kernel(const float* const* __restrict__ Aarray, int n, int lda, cons
         }
     }
     __syncthreads();
-    const int c0 = ((int)blockIdx.y * (threads >> 5) + warp) * CW;  // this warp's right-hand sides
-    const bool work = c0 < nrhs;
+    const long long c0l = first + ((long long)blockIdx.y * (threads >> 5) + warp) * CW;
+    const bool work = c0l < nrhs;
+    const int c0 = work ? (int)c0l : nrhs;  // this warp's right-hand sides
     float2 p[R][CW / 2];
     int row[R];
 #pragma unroll
@@ -104,13 +106,17 @@ template <int R, int CW>
 static cudaError_t launch_block(cudaStream_t st, int n, int nrhs, const float* const* Aarray, int lda, const int* ipiv,
                                 float* const* Barray, int ldb, int batch)
 {
-    const int blocks = (nrhs + CW - 1) / CW;
+    const int blocks = (int)((nrhs + (long long)CW - 1) / CW);
     const int parts = (blocks + kGbMaxWarps - 1) / kGbMaxWarps, warps = (blocks + parts - 1) / parts;
     const size_t smem = (size_t)(2 * kSvNB * (32 * R + 4) + warps * kSvNB * kSvULd<CW> + 2 * 32 * R) * 4;
     const cudaError_t e = ensure_smem_limit(getrs_block_kernel<R, CW>, 64 * 1024);
     if (e != cudaSuccess) return e;
-    getrs_block_kernel<R, CW><<<dim3((unsigned)batch, (unsigned)parts), warps * 32, smem, st>>>(Aarray, n, lda, ipiv,
-                                                                                               Barray, ldb, nrhs);
+    // one launch for as many CTAs a matrix as a grid's second dimension takes
+    for (int p0 = 0; p0 < parts; p0 += kMaxGridY) {
+        const dim3 grid((unsigned)batch, (unsigned)std::min(parts - p0, kMaxGridY));
+        getrs_block_kernel<R, CW><<<grid, warps * 32, smem, st>>>(Aarray, n, lda, ipiv, Barray, ldb, nrhs,
+                                                                  p0 * warps * CW);
+    }
     return cudaGetLastError();
 }
 

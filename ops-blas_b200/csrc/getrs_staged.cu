@@ -281,7 +281,7 @@ template <int MODE>
 __global__ void __launch_bounds__(kSgThreads)
 getrs_staged_kernel(const float* const* __restrict__ Aarray, int n, int lda, const int* __restrict__ ipiv,
                     float* const* __restrict__ Barray, int ldb, int nrhs, int batch, int n8, int region, int xs,
-                    int per, int cols)
+                    int per, int cols, int first)
 {
     constexpr bool TR = MODE == 1;
     constexpr int WARPS = kSgThreads / 32;
@@ -290,7 +290,7 @@ getrs_staged_kernel(const float* const* __restrict__ Aarray, int n, int lda, con
     int* pv = reinterpret_cast<int*>(xall + per * cols * xs);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long m0 = (long long)blockIdx.x * per;
-    const int c0 = (int)blockIdx.y * cols, cw = min(cols, nrhs - c0);
+    const int c0 = first + (int)blockIdx.y * cols, cw = min(cols, nrhs - c0);
 
     // LU of the CTA's matrices on its way; those without a right-hand side (NULL) are skipped
     for (int g = 0; g < per; g++) {
@@ -401,9 +401,13 @@ cudaError_t getrs_staged_launch(cudaStream_t st, bool trans, int n, int nrhs, co
                             : getrs_staged_kernel<4>;
     const cudaError_t e = ensure_smem_limit(kernel, 200 * 1024);
     if (e != cudaSuccess) return e;
-    const dim3 grid((unsigned)((batch + (long long)s.per - 1) / s.per), (unsigned)((nrhs + s.cols - 1) / s.cols));
-    kernel<<<grid, kSgThreads, s.smem, st>>>(Aarray, n, lda, ipiv, Barray, ldb, nrhs, batch, s.n8, s.region, s.xs,
-                                             s.per, s.cols);
+    // one launch for as many column blocks as a grid's second dimension takes
+    for (long long first = 0; first < nrhs; first += (long long)kMaxGridY * s.cols) {
+        const long long blocks = std::min<long long>((nrhs - first + s.cols - 1) / s.cols, kMaxGridY);
+        const dim3 grid((unsigned)((batch + (long long)s.per - 1) / s.per), (unsigned)blocks);
+        kernel<<<grid, kSgThreads, s.smem, st>>>(Aarray, n, lda, ipiv, Barray, ldb, nrhs, batch, s.n8, s.region, s.xs,
+                                                 s.per, s.cols, (int)first);
+    }
     return cudaGetLastError();
 }
 

@@ -51,6 +51,8 @@ unsigned wait_limit(unsigned def);
 // Number of SMs of the current device (cached per device).
 int sm_count();
 
+constexpr int kMaxGridY = 65535;  // blocks of a grid's second dimension
+
 // Raises a kernel's dynamic shared-memory limit to at least `bytes` on the current device. The
 // attribute is per device, so the set-up is remembered per (device, kernel) under a lock; the
 // result of cudaFuncSetAttribute is returned (a cached success afterwards). The record does not

@@ -38,3 +38,44 @@ def test_getrs_many_rhs_trans_n(handle, n, nrhs, batch, pad):
     keep[np.arange(0, batch, 97)] = False
     assert_bitwise(got[keep], want[keep], f"n={n} nrhs={nrhs}")
     assert np.array_equal(got[~keep], b[~keep])
+
+
+def test_refine_more_columns_than_one_grid_takes(ob, cuda):
+    """n <= 128: the solve's blocks of right-hand sides are a grid's second dimension (65535 of them at most)."""
+    import torch
+
+    n, k = 33, 64
+    nrhs = (65536 * 128 // k + 1) * k
+    g = torch.Generator(device="cuda").manual_seed(1)
+    A = torch.randn(1, n, n, device="cuda", generator=g) + 12 * torch.eye(n, device="cuda")
+    B = torch.randn(k, n, device="cuda", generator=g).repeat(nrhs // k, 1).reshape(1, nrhs, n)
+    few = B[:, :k].clone()
+    with ob.Handle() as h:  # its own: the workspace of this call is a gigabyte
+        X, LU, piv, info, _, _ = h.refine(A, B, n, nrhs, max_iter=0, compute=ob.COMPUTE_32F)
+        h.getrs("N", LU, n, n, piv, few, k, n)
+        torch.cuda.synchronize()
+    assert int(info[0]) == 0
+    assert torch.equal(X.reshape(nrhs // k, k, n), few.expand(nrhs // k, k, n))
+
+
+def test_grouped_more_columns_than_one_grid_takes(ob, handle):
+    """128 < n <= 256, as above through a plan (whose groups above 128 run on the batched kernels)."""
+    import torch
+
+    n, k = 129, 64
+    nrhs = 65536 * 64 + k
+    g = torch.Generator(device="cuda").manual_seed(2)
+    A = torch.randn(1, n, n, device="cuda", generator=g) + 24 * torch.eye(n, device="cuda")
+    B = torch.randn(k, n, device="cuda", generator=g).repeat(nrhs // k, 1).reshape(1, nrhs, n)
+    few = B[:, :k].clone()
+    LU = A.clone()
+    piv, _ = handle.getrf(LU, n, n)
+    handle.getrs("N", LU, n, n, piv, few, k, n)
+    piv = torch.empty(n, dtype=torch.int32, device="cuda")
+    info = torch.empty(1, dtype=torch.int32, device="cuda")
+    with_plan = ob.GroupedPlan(handle, [n], [nrhs], [1])
+    with_plan.run(handle, ob.ptr_array(A), piv, info, ob.ptr_array(B))
+    torch.cuda.synchronize()
+    with_plan.close()
+    assert int(info[0]) == 0
+    assert torch.equal(B.reshape(nrhs // k, k, n), few.expand(nrhs // k, k, n))
