@@ -333,27 +333,25 @@ gels_warp_kernel(int trans, int m, int n, int nrhs, float* const* __restrict__ A
 
 // QR-path systems beyond the warp kernel that fit shared memory: one a CTA, a warp per 64 columns, the
 // right-hand sides as further columns (qr_smem.cuh), then a thread per right-hand side for R x = c.
-// 48 x 30 with 4 right-hand sides x 4096: 1031 us in global memory, 202 here; 40 x 10, 2 x 8192: 349, 128.
+// us, in global memory -> here: 64 x 48 with 4 right-hand sides x 2048 2054 -> 205; 40 x 10, 2 x 8000
+// 324 -> 116; 33 x 4, 30 x 148 20 -> 16.
 __global__ void __launch_bounds__(128)
 gels_smem_kernel(int trans, int m, int n, int nrhs, float* const* __restrict__ Aarray, int lda,
                  float* const* __restrict__ Carray, int ldc, int* __restrict__ info)
 {
     extern __shared__ __align__(16) float dyn[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+    const int tid = threadIdx.x, warps = blockDim.x >> 5;
     const int rows = trans ? n : m, N = trans ? m : n, cols = N + nrhs;
     const QsSmem M(dyn, rows, cols);
     float* A = Aarray[blockIdx.x];
     float* C = Carray[blockIdx.x];
-    if (trans) {
-        for (int r = warp; r < rows; r += warps)
-            for (int c = lane; c < N; c += 32) M.a[r * M.ld + c] = A[c + (long long)r * lda];
-    } else {
-        for (int c = warp; c < N; c += warps)
-#pragma unroll 4
-            for (int r = lane; r < rows; r += 32) M.a[r * M.ld + c] = A[r + (long long)c * lda];
-    }
-    for (int j = warp; j < nrhs; j += warps)
-        for (int r = lane; r < rows; r += 32) M.a[r * M.ld + N + j] = C[r + (long long)j * ldc];
+    if (trans)
+        qs_columns(N, rows, warps * 32, tid, [&](int c, int r) { cp_async4(M.a + r * M.ld + c, A + c + (long long)r * lda); });
+    else
+        qs_columns(rows, N, warps * 32, tid, [&](int r, int c) { cp_async4(M.a + r * M.ld + c, A + r + (long long)c * lda); });
+    qs_columns(rows, nrhs, warps * 32, tid,
+               [&](int r, int j) { cp_async4(M.a + r * M.ld + N + j, C + r + (long long)j * ldc); });
+    cp_async_wait_all();
     qs_sync(warps);
     qs_factor<true>(
         M, rows, N, cols, warps, tid,
@@ -372,9 +370,7 @@ gels_smem_kernel(int trans, int m, int n, int nrhs, float* const* __restrict__ A
         [](float x, float sc) { return __fmul_rn(x, sc); }, [](int, float) {});
     // factors back (trans: the n x m transpose with leading dimension n, as the reference leaves it)
     const int ldo = trans ? rows : lda;
-    for (int c = warp; c < N; c += warps)
-#pragma unroll 4
-        for (int r = lane; r < rows; r += 32) A[r + (long long)c * ldo] = M.a[r * M.ld + c];
+    qs_columns(rows, N, warps * 32, tid, [&](int r, int c) { A[r + (long long)c * ldo] = M.a[r * M.ld + c]; });
     // the highest zero diagonal stops the first right-hand side there and leaves the others
     int stop = -1;
     for (int i = N - 1; i >= 0 && stop < 0; i--)
@@ -390,8 +386,7 @@ gels_smem_kernel(int trans, int m, int n, int nrhs, float* const* __restrict__ A
         }
     }
     qs_sync(warps);
-    for (int j = warp; j < nrhs; j += warps)
-        for (int r = lane; r < rows; r += 32) C[r + (long long)j * ldc] = M.a[r * M.ld + N + j];
+    qs_columns(rows, nrhs, warps * 32, tid, [&](int r, int j) { C[r + (long long)j * ldc] = M.a[r * M.ld + N + j]; });
     if (tid == 0) info[blockIdx.x] = stop >= 0 ? stop + 1 : 0;
 }
 

@@ -111,19 +111,18 @@ geqrf_col_kernel(float* const* __restrict__ Aarray, int n, int lda, float* const
 }
 
 // Larger shapes that fit shared memory: one matrix a CTA, a warp per 64 columns (qr_smem.cuh). Bound by
-// instruction issue and the row-order sums. 64 x 48 x 4096: 377 us, the generic kernel's thread-0
-// reflector over global memory 3550; 40 x 33 x 4096: 156 and 550; 200 x 200 x 148: 912 and 3680.
+// instruction issue and the row-order sums. us, the generic kernel's thread-0 reflector over global memory
+// -> this: 64 x 48 x 4096 3542 -> 297, 33 x 33 x 148 55 -> 45, 33 x 33 x 4096 365 -> 103.
 __global__ void __launch_bounds__(128)
 geqrf_smem_kernel(float* const* __restrict__ Aarray, int m, int n, int lda, float* const* __restrict__ TauArray)
 {
     extern __shared__ __align__(16) float dyn[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+    const int tid = threadIdx.x, warps = blockDim.x >> 5;
     const QsSmem M(dyn, m, n);
     float* A = Aarray[blockIdx.x];
     float* tau = TauArray[blockIdx.x];
-    for (int c = warp; c < n; c += warps)
-#pragma unroll 4
-        for (int r = lane; r < m; r += 32) M.a[r * M.ld + c] = A[r + (long long)c * lda];
+    qs_columns(m, n, warps * 32, tid, [&](int r, int c) { cp_async4(M.a + r * M.ld + c, A + r + (long long)c * lda); });
+    cp_async_wait_all();
     qs_sync(warps);
     qs_factor<false>(
         M, m, m < n ? m : n, n, warps, tid,
@@ -136,9 +135,7 @@ geqrf_smem_kernel(float* const* __restrict__ Aarray, int m, int n, int lda, floa
             return t != 0.0f;
         },
         [](float x, float sc) { return __fdiv_rn(x, sc); }, [&](int i, float t) { tau[i] = t; });
-    for (int c = warp; c < n; c += warps)
-#pragma unroll 4
-        for (int r = lane; r < m; r += 32) A[r + (long long)c * lda] = M.a[r * M.ld + c];
+    qs_columns(m, n, warps * 32, tid, [&](int r, int c) { A[r + (long long)c * lda] = M.a[r * M.ld + c]; });
 }
 
 constexpr int kQrThreads = 256;

@@ -7,6 +7,8 @@
 
 #include <cuda_runtime.h>
 
+#include "small_common.cuh"
+
 namespace opsblas {
 
 constexpr int kQsMaxCols = 256;  // four warps
@@ -40,6 +42,27 @@ __device__ __forceinline__ void qs_sync(int warps)
         __syncwarp();
     else
         __syncthreads();
+}
+
+// f(r, c) for every element of m rows and n columns, column after column over the CTA's threads, so that a
+// warp is full on any number of rows and a thread's elements do not wait for each other (a warp a column,
+// each load waiting for its store, left few columns on their way and few lanes at work: us, geqrf
+// 33 x 33 x 148 64 -> 45, 64 x 48 x 4096 377 -> 297, 1 x 64 x 148 23 -> 6).
+template <class F>
+__device__ __forceinline__ void qs_columns(int m, int n, int threads, int tid, F f)
+{
+    const int dr = threads % m, dc = threads / m;
+    int r = tid % m, c = tid / m;
+#pragma unroll 4
+    for (int e = tid; e < m * n; e += threads) {
+        f(r, c);
+        r += dr;
+        c += dc;
+        if (r >= m) {
+            r -= m;
+            c++;
+        }
+    }
 }
 
 // Applies the reflector (v rows i+1 .., t) to this lane's columns c0 and c0 + 32 (those in (i, cols)) and
