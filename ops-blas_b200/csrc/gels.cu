@@ -459,7 +459,9 @@ extern "C" aclblasStatus_t aclblasSgelsBatched(aclblasHandle_t handle, aclblasOp
                   kGelsMaxSmem / 4, lda, n);
         return ACLBLAS_STATUS_NOT_SUPPORTED;
     }
-    if (effM >= effN && qs_supported(effM, effN + nrhs)) {
+    // one reflector is worth the way through shared memory once every SM has a matrix (us, global and shared:
+    // 33 x 1 with 16 right-hand sides x 1 8 and 10, 33 x 1 with 8 x 148 10 and 10, with 100 x 148 21 and 12)
+    if (effM >= effN && (effN > 1 || batchSize >= sm_count()) && qs_supported(effM, effN + nrhs)) {
         const cudaError_t e = ensure_smem_limit(gels_smem_kernel, kQsMaxBytes);
         if (e != cudaSuccess) return launch_status(kApi, e);
         gels_smem_kernel<<<(unsigned)batchSize, qs_warps(effN + nrhs) * 32, qs_bytes(effM, effN + nrhs),

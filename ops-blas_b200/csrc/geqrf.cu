@@ -13,7 +13,7 @@
 //   m, n <= 32 : geqrf_col_kernel<M>, one warp per matrix, lane c = column c in registers (every
 //                sum local, in row order), the reflector published through shared memory with
 //                its divisions one row per lane, the column update in packed f32x2 operations;
-//   n <= 256 and the matrix in shared memory: geqrf_smem_kernel, a warp per 64 columns;
+//   1 < n <= 256, m > 1 and the matrix in shared memory: geqrf_smem_kernel, a warp per 64 columns;
 //   otherwise  : geqrf_generic_kernel, one CTA per matrix in global memory (correctness path):
 //                thread 0 forms the reflector, thread t updates columns i+1+t, i+1+t+256, ...
 #include <cuda_runtime.h>
@@ -253,7 +253,9 @@ extern "C" aclblasStatus_t aclblasSgeqrfBatched(aclblasHandle_t handle, int m, i
             default:
                 break;
         }
-    } else if (qs_supported(m, n)) {
+    } else if (m > 1 && n > 1 && qs_supported(m, n)) {
+        // one reflector is not worth the way through shared memory (us, generic and this: 33 x 1 x 148 6 and 8,
+        // 100 x 1 x 8000 31 and 37; 33 x 2 x 8000 47 and 27)
         const cudaError_t e = ensure_smem_limit(geqrf_smem_kernel, kQsMaxBytes);
         if (e != cudaSuccess) return launch_status(kApi, e);
         geqrf_smem_kernel<<<(unsigned)batchSize, qs_warps(n) * 32, qs_bytes(m, n), st>>>(Aarray, m, n, lda, TauArray);

@@ -23,7 +23,7 @@ def _members(rng, shape, m):
     return a
 
 
-@pytest.mark.parametrize("mn", [(33, 1), (1, 33), (33, 32), (32, 33), (64, 48), (47, 64), (65, 65), (64, 66), (40, 128),
+@pytest.mark.parametrize("mn", [(33, 1), (1, 33), (33, 2), (2, 33), (33, 32), (32, 33), (64, 48), (47, 64), (65, 65), (64, 66), (40, 128),
                                 (129, 40), (30, 129), (35, 193), (20, 256), (20, 257), (222, 222), (256, 200)])
 def test_geqrf_smem_edges(handle, mn):
     m, n = mn
@@ -31,6 +31,16 @@ def test_geqrf_smem_edges(handle, mn):
         a = _members(np.random.default_rng(m * 300 + n), (7, n, lda), m)
         with np.errstate(all="ignore"):
             check_geqrf(handle, a, m, n, lda, f"{m}x{n} lda {lda}")
+
+
+@pytest.mark.parametrize("batch", [7, 200])
+def test_gels_one_column(handle, batch):
+    """One reflector: in global memory for a small batch, in shared memory for one that fills the GPU."""
+    rng = np.random.default_rng(batch)
+    a = _members(rng, (batch, 1, 33), 33)
+    c = rng.standard_normal((batch, 20, 33)).astype(np.float32)
+    with np.errstate(all="ignore"):
+        check_gels(handle, "N", a, c, 33, 1, 20, 33, 33, f"33x1 batch {batch}")
 
 
 @pytest.mark.parametrize("shape", [("N", 33, 32, 1), ("N", 64, 48, 15), ("N", 64, 48, 17), ("T", 48, 64, 1),
