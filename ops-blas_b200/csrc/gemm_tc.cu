@@ -4,8 +4,8 @@
 //   offsets a_off / b_off / c_off added to every matrix pointer)
 //
 // Persistent: one CTA per SM walks the 128 x 128 tiles of C (one contiguous range of tiles per CTA where
-// everything goes by TMA, so that consecutive tiles keep their matrix's tensor maps; else tile t,
-// t + #CTAs, ...), nine warps:
+// everything goes by TMA and a matrix has several, so that consecutive tiles keep their matrix's tensor
+// maps; else tile t, t + #CTAs, ...), nine warps:
 //   * warps 0-3 produce: per K tile (128 bytes of K: 64 FP16/BF16, 128 FP8 or 32 TF32 values) they
 //     fill a stage of a ring that runs across tile boundaries with op(A) rows m0..m0+127 and
 //     op(B)^T rows n0..n0+127 in the 128-byte swizzled canonical UMMA layout of the operand's
@@ -645,7 +645,6 @@ gemm_tc_kernel(int M, int N, int K, float alpha, const void* const* __restrict__
         long long g = 0;          // K tiles issued by this CTA (the ring position)
         long long issued = 0;     // K tiles whose loads were actually issued (warp 0 tracks it)
         long long mapped = -1;    // the matrix the global maps point at
-        const void *pre_a = nullptr, *pre_b = nullptr;  // the next tile's matrix pointers, read ahead
         for (long long t = t_first; t < t_last; t += t_step) {
             // every producer thread takes the same path through every tile (named barrier 1)
             if (producers_any(aborted())) break;
@@ -653,15 +652,8 @@ gemm_tc_kernel(int M, int N, int K, float alpha, const void* const* __restrict__
             int tile;
             tile_split(t, tiles, bidx, tile);
             const int m0 = (tile % tiles_m) * kTcTile, n0 = (tile / tiles_m) * kTcTile;
-            const SA* A = static_cast<const SA*>(t == t_first ? Aarr[bidx] : pre_a) + a_off;
-            const SB* B = static_cast<const SB*>(t == t_first ? Barr[bidx] : pre_b) + b_off;
-            if (t + t_step < t_last) {  // the next tile's matrices: the latency hides behind this tile
-                long long bnx;
-                int tlx;
-                tile_split(t + t_step, tiles, bnx, tlx);
-                pre_a = Aarr[bnx];
-                pre_b = Barr[bnx];
-            }
+            const SA* A = static_cast<const SA*>(Aarr[bidx]) + a_off;
+            const SB* B = static_cast<const SB*>(Barr[bidx]) + b_off;
             const bool avec = (reinterpret_cast<uintptr_t>(A) & 15) == 0 && ((long long)lda * ES) % 16 == 0;
             const bool bvec = (reinterpret_cast<uintptr_t>(B) & 15) == 0 && ((long long)ldb * ES) % 16 == 0;
             const bool tma = use_tma && avec && bvec;
@@ -1172,10 +1164,12 @@ static cudaError_t tc_launch_t(cudaStream_t st, bool transA, bool transB, int m,
     // the TMA epilogue: beta = 0 stores alpha * D, otherwise loads C, combines and stores
     int epi_mode = beta == 0.0f ? 1 : 2;
     if (epi_mode != 0 && !(slots && tmap_encode_c<TC>(&mc, tmslots, m, n, ldc))) epi_mode = 0;
-    // One contiguous range of tiles a CTA where operands and C go by TMA: a matrix's maps are then set up
-    // once for its tiles (BF16 256^3 x 2048: 183 us, against 220 with every gridDim.x-th tile). Without
-    // maps to keep the interleaved order balances better (FP16 201 x 121 x 89 x 1024: 258, 275 us).
-    const int contig = LU || (use_tma && epi_mode != 0) ? 1 : 0;
+    // One contiguous range of tiles a CTA where operands and C go by TMA and a matrix has several tiles: its
+    // maps are then set up once for them (us, every gridDim.x-th tile and this: BF16 256^3 x 1000 107 and 92,
+    // with beta 0.5 135 and 123; TF32 T N 256 x 256 x 32 x 1000 147 and 123). With a tile a matrix, or without
+    // maps to keep, the interleaved order balances better (TF32 T N 64^3 x 4000: 182, 186; FP16
+    // 201 x 121 x 89 x 1024: 258, 275).
+    const int contig = LU || (use_tma && epi_mode != 0 && tm * tn > 1) ? 1 : 0;
     gemm_tc_kernel<TA, TB, TC, SPLIT, LU><<<(unsigned)grid, kTcThreads, smem, st>>>(
         m, n, k, alpha, A, a_off, lda, transA ? 1 : 0, B, b_off, ldb, transB ? 1 : 0, beta, C, c_off, ldc, tm, tn,
         total, status, wait_limit(kTcWaitPolls), ma, mb, static_cast<CUtensorMap*>(tmslots), use_tma ? 1 : 0,

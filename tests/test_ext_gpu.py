@@ -105,6 +105,24 @@ def test_gemm_batched_ex_numerics(handle, case):
         assert np.max(err / scale) <= rtol, np.max(err / scale)
 
 
+@pytest.mark.parametrize("m,n", [(128, 128), (136, 64), (256, 256)])
+@pytest.mark.parametrize("beta", [0.0, 0.5])
+def test_gemm_tiles_of_many_matrices(handle, m, n, beta):
+    """More tiles than SMs, with one, two and four tiles a matrix: every tile once, in both orders of the tiles.
+    One rounding of the BF16 result (2^-8 of its value) and FP32 sums of k = 72 products."""
+    import torch
+
+    batch, k = 333, 72
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    A = torch.randn(batch, m, k, device="cuda", generator=g).bfloat16()  # transposed: K contiguous
+    B = torch.randn(batch, n, k, device="cuda", generator=g).bfloat16()
+    Cm = torch.randn(batch, n, m, device="cuda", generator=g).bfloat16()
+    ref = torch.einsum("bmk,bnk->bnm", A.double(), B.double()) + beta * Cm.double()
+    handle.gemm_batched_ex("T", "N", m, n, k, 1.0, A, DT["BF16"], k, B, DT["BF16"], k, beta, Cm, DT["BF16"], m)
+    err = (Cm.double() - ref).abs()
+    assert torch.all(err <= 2.0 ** -8 * ref.abs() + 72 * 2.0 ** -23 * 8)
+
+
 def test_gemm_batched_ex_early_exit(handle):
     """k == 0 or alpha == 0: C = beta * C; beta == 1 leaves C untouched; beta == 0 writes zeros."""
     import torch
