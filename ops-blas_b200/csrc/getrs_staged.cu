@@ -10,7 +10,7 @@
 // Bound by latency at the 12 matrices (n = 64) to 3 (n = 128) that an SM's shared memory holds. B200,
 // CUDA events, us, before (a thread per right-hand side reading LU through L1, or a CTA of 256 threads
 // for one matrix) -> now: N, n = 64, 8 columns x 65536: 1670 -> 905; n = 100, 1 x 4096: 365 -> 127;
-// n = 128, 16 x 4096: 1612 -> 433, 8 x 4096: 419 -> 419; T, n = 64, 8 x 65536: 1551 -> 1200; n = 100,
+// n = 128, 16 x 4096: 1610 -> 422, 100 x 600: 498 -> 365; T, n = 64, 8 x 65536: 1551 -> 1200; n = 100,
 // 1 x 4096: 847 -> 309.
 // Every element takes one fmaf per term in the reference's order and is divided as there, so the
 // results are its bits. Rows and columns past n are zero: -0 * 0 added to a sum leaves it as it is.
@@ -38,7 +38,11 @@ struct SgShape {
         n8 = (n + 7) & ~7;
         region = n8 * n8 + 4;  // odd in 16-byte units: the matrices of a warp are read from different banks
         xs = n8 + 4;
-        cols = std::min(nrhs, kSgThreads);
+        // equal blocks of at most 32 columns, a CTA each: with 128 in one, x takes as much shared memory as
+        // LU and an SM holds one CTA (us, n = 128, 128 columns x 300: N 442 -> 205, T 737 -> 328;
+        // n = 33, T, 128 x 1: 70 -> 25)
+        const int blocks = (nrhs + 31) / 32;
+        cols = (nrhs + blocks - 1) / blocks;
         const int bytes = (region + n8 + cols * xs) * 4;
         per = std::max(1, std::min(32 / cols, kSgBudget / bytes));
         per = std::max(1, std::min(per, batch / (3 * sm_count())));  // a small batch spreads over the SMs first
@@ -350,22 +354,20 @@ getrs_staged_kernel(const float* const* __restrict__ Aarray, int n, int lda, con
     if constexpr (MODE < 2) {
         // lane = right-hand side, in every warp alike
         const int g = lane / cw, c = lane - g * cw;
-        for (int cc = 0; cc < cw; cc += 32) {  // (more than 32 columns: one matrix, 32 at a time)
-            const bool work = lane < per * cw && c + cc < cw && m0 + g < batch && Barray[m0 + g] != nullptr;
-            const float* m = sm + (work ? g : 0) * region;
-            float* x = xall + (work ? g * cols + c + cc : 0) * xs;
-            const int* p = pv + (work ? g : 0) * n8;
-            if (TR) {
-                sg_sweep<SgTri::UPPER_T>(m, n8, x, n, warp, work);
-                if (warp == ((cc >> 5) & 3) && work) {
-                    sg_lower_t(m, n8, x, n);
-                    sg_interchange<true>(x, p, n8);
-                }
-            } else {
-                if (warp == 0 && work) sg_interchange<false>(x, p, n8);
-                sg_sweep<SgTri::LOWER>(m, n8, x, n, warp, work);
-                sg_sweep<SgTri::UPPER>(m, n8, x, n, warp, work);
+        const bool work = lane < per * cw && m0 + g < batch && Barray[m0 + g] != nullptr;
+        const float* m = sm + (work ? g : 0) * region;
+        float* x = xall + (work ? g * cols + c : 0) * xs;
+        const int* p = pv + (work ? g : 0) * n8;
+        if (TR) {
+            sg_sweep<SgTri::UPPER_T>(m, n8, x, n, warp, work);
+            if (warp == 0 && work) {
+                sg_lower_t(m, n8, x, n);
+                sg_interchange<true>(x, p, n8);
             }
+        } else {
+            if (warp == 0 && work) sg_interchange<false>(x, p, n8);
+            sg_sweep<SgTri::LOWER>(m, n8, x, n, warp, work);
+            sg_sweep<SgTri::UPPER>(m, n8, x, n, warp, work);
         }
     } else {
         for (int v = warp; v < per * cw; v += WARPS) {
