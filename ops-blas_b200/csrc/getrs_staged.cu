@@ -296,6 +296,9 @@ getrs_staged_kernel(const float* const* __restrict__ Aarray, int n, int lda, con
     const long long m0 = (long long)blockIdx.x * per;
     const int c0 = first + (int)blockIdx.y * cols, cw = min(cols, nrhs - c0);
 
+    bool any = false;
+    for (int g = 0; g < per; g++) any |= m0 + g < batch && Barray[m0 + g] != nullptr;
+    if (!any) return;  // nothing to solve (a refinement's converged matrices), for the whole CTA
     // LU of the CTA's matrices on its way; those without a right-hand side (NULL) are skipped
     for (int g = 0; g < per; g++) {
         if (m0 + g >= batch || Barray[m0 + g] == nullptr) continue;
