@@ -9,7 +9,8 @@
 //   n <= 32, otherwise : getrs_rhs_kernel, one lane per right-hand side, LU staged in shared
 //                        memory by cp.async;
 //   32 < n <= 128      : getrs_staged_kernel (getrs_staged.cu), LU staged in shared memory, a lane per
-//                        right-hand side, or a warp for one of few;
+//                        right-hand side, or a warp for one of few; a few columns of n = 96 and 128 in
+//                        small batches go to getrs_blk_kernel (getrs_blk_preferred);
 //   128 < n <= 256, N   : getrs_block_kernel (getrs_block.cu), right-hand sides in registers, when there are
 //                        enough of them; otherwise as n > 256;
 //   n > 256, trans N   : getrs_blk_kernel (getrs_blk.cu), blocked, right-hand sides in shared memory;
@@ -130,6 +131,8 @@ cudaError_t getrs_launch(cudaStream_t st, bool tr, int n, int nrhs, const float*
             getrs_small_dispatch_t(n, st, Aarray, lda, devIpiv, Barray, ldb, nrhs, batchCount);
         else
             getrs_small_dispatch_n(n, st, Aarray, lda, devIpiv, Barray, ldb, nrhs, batchCount);
+    } else if (!tr && getrs_blk_preferred(n, nrhs, batchCount)) {
+        return getrs_blk_launch(st, n, nrhs, Aarray, lda, devIpiv, Barray, ldb, batchCount);
     } else if (getrs_staged_supported(n)) {
         return getrs_staged_launch(st, tr, n, nrhs, Aarray, lda, devIpiv, Barray, ldb, batchCount);
     } else if (!tr && getrs_block_preferred(n, nrhs, batchCount)) {

@@ -1,4 +1,4 @@
-// aclblasSgetrsBatched, trans N, n > 128: one CTA per matrix, blocked substitution with the
+// aclblasSgetrsBatched, trans N, n > 128 (and few columns of n = 96, 128): one CTA per matrix, blocked substitution with the
 // right-hand sides resident in shared memory.
 //
 // The reference solve (sgetrs_batched_kernel.cpp:83-200) is laswp, then the unit-L forward sweep
@@ -284,6 +284,14 @@ getrs_blk_kernel(const float* const* __restrict__ Aarray, int n, int lda, const 
         }
         __syncthreads();
     }
+}
+
+// 32 < n <= 128: whole blocks of 32 rows and one pass over the columns, in batches that leave SMs idle, are a
+// little faster here than staged (us, staged and here: n = 128, 8 columns x 16 37, 35, x 600 84, 78,
+// x 1500 166, 168; n = 96, 16 x 148 31, 29, x 600 41, 57; n = 64, 8 x 148 21, 21; n = 100, 8 x 148 33, 33).
+bool getrs_blk_preferred(int n, int nrhs, int batch)
+{
+    return n > 64 && n <= 128 && n % kBsB == 0 && nrhs > 2 && nrhs <= kBsRC && batch <= (n > 96 ? 5 : 2) * sm_count();
 }
 
 bool getrs_blk_supported(int n) { return n > 32 && getrs_blk_smem(n) <= 200 * 1024; }
