@@ -96,12 +96,15 @@ getrs_block_kernel(const float* const* __restrict__ Aarray, int n, int lda, cons
     }
 }
 
-// A warp per 16 right-hand sides needs enough of them to hide its latency: with fewer than two an SM the
-// CTA of 256 threads for one matrix (getrs_blk.cu) is faster (us, n = 200, 8 columns x 148: 135 here, 69
-// there; n = 256, 40 x 148: 145, 207; 4 x 512: 116, 190; 16 x 2048: 421, 532; 1 x 2048: 430, 511).
+// A warp per 16 right-hand sides needs enough of them to hide its latency. Up to 16 columns are one pass of
+// the CTA of 256 threads for one matrix (getrs_blk.cu), three of which an SM holds: that is faster until a
+// second wave of them (us, there and here: n = 160, 8 columns x 300 59, 82, x 500 96, 82; n = 256,
+// 16 x 444 121, 133, x 500 190, 135). More columns are passes in turn there: here from two warps an SM on
+// (n = 129, 17 x 148 80, 59; n = 256, 40 x 148 207, 145).
 bool getrs_block_preferred(int n, int nrhs, int batch)
 {
-    return n > 128 && n <= 256 && (long long)batch * ((nrhs + 15) / 16) >= 2 * sm_count();
+    if (n <= 128 || n > 256) return false;
+    return nrhs <= 16 ? batch > 3 * sm_count() : (long long)batch * ((nrhs + 15) / 16) >= 2 * sm_count();
 }
 
 template <int R, int CW>

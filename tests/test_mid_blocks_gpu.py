@@ -121,7 +121,7 @@ def test_getrs_block_edges(handle, n):
     """The register solve (getrs_block.cu): panel and tile edges, column counts around 4, 16 and a CTA's 64, odd
     strides, invalid pivots, a zero on the diagonal, infinities and NaN."""
     rng = np.random.default_rng(n)
-    for nrhs, batch, pad in ((1, 300, 0), (4, 300, 1), (5, 300, 4), (16, 3, 0), (17, 160, 0), (70, 60, 3)):
+    for nrhs, batch, pad in ((1, 460, 0), (4, 460, 1), (5, 460, 4), (16, 3, 0), (17, 160, 0), (70, 60, 3)):
         ld = n + pad
         lu = rng.standard_normal((batch, n, ld)).astype(np.float32)
         lu[:, np.arange(n), np.arange(n)] += 12
