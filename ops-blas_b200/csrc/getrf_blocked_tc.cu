@@ -33,6 +33,7 @@
 #include "f32x2.cuh"
 #include "internal.h"
 #include "lu_mid.cuh"
+#include "quotient.cuh"
 #include "small_common.cuh"
 #include "tc_common.cuh"
 
@@ -209,14 +210,13 @@ __device__ __forceinline__ void bp_take_row(f32x2 (&p)[kBpH / 2], const float* s
 // Factors hw columns (k .. of half h) of the panel held in p: one CTA barrier per column. Each warp finds
 // its first maximum (two redux), publishes magnitude, position and the row; after the barrier every
 // warp takes the best of the warps' (two redux) and reads the pivot row. Returns the columns eliminated.
-// Multipliers are correctly rounded quotients by one reciprocal, and a row that has become a pivot is
-// poisoned with NaN until the half is done (both as in lu_mid.cuh: masks cost more than the updates).
+// Multipliers are correctly rounded quotients by one reciprocal (quotient.cuh), and a row that has become a
+// pivot is poisoned with NaN until the half is done (as in lu_mid.cuh: masks cost more than the updates).
 template <int NT, int RPT, bool PIVOT>
 __device__ __forceinline__ int lu_panel_half(f32x2 (&p)[RPT][kBpH / 2], int (&pos)[RPT], BpSmem<NT / 32>& S, int k,
                                              int hw, int* __restrict__ piv, int tid, int warp, int lane)
 {
     constexpr int NW = NT / 32;
-    constexpr float lo = 0x1p-60f, hi = 0x1p60f;
     int done = hw;
 #pragma unroll
     for (int c = 0; c < kBpH; c++, k++) {
@@ -256,8 +256,8 @@ __device__ __forceinline__ int lu_panel_half(f32x2 (&p)[RPT][kBpH / 2], int (&po
             ppos = (int)__reduce_min_sync(0xffffffffu, sl.x == g ? sl.y : 0x7fffffffu);
             bw = __ffs(__ballot_sync(0xffffffffu, sl.y == (unsigned)ppos)) - 1;
             const float mx = __uint_as_float(g);
-            y = mid_reciprocal(mx);
-            usual = mx >= lo && mx <= hi;
+            y = qt_reciprocal(mx);
+            usual = qt_usual(mx);
         } else {  // the row at position k, published by its warp
 #pragma unroll
             for (int r = 0; r < RPT; r++)
@@ -289,20 +289,12 @@ __device__ __forceinline__ int lu_panel_half(f32x2 (&p)[RPT][kBpH / 2], int (&po
             done = c;
             break;
         }
-        y = copysignf(y, pv);
         float l[RPT];
-        float least = fabsf(a[0]);
+        if (PIVOT) {
+            qt_quotients<RPT>(a, pv, copysignf(y, pv), usual, l);
+        } else {
 #pragma unroll
-        for (int r = 0; r < RPT; r++) {
-            if (r > 0) least = fminf(least, fabsf(a[r]));
-            l[r] = __fmul_rn(a[r], y);
-            l[r] = fmaf(fmaf(-l[r], pv, a[r]), y, l[r]);
-            l[r] = fmaf(fmaf(-l[r], pv, a[r]), y, l[r]);
-        }
-        if (!usual || least < lo) {
-#pragma unroll
-            for (int r = 0; r < RPT; r++)
-                if (!usual || fabsf(a[r]) < lo) l[r] = a[r] / pv;
+            for (int r = 0; r < RPT; r++) l[r] = a[r] / pv;
         }
 #pragma unroll
         for (int r = 0; r < RPT; r++) {

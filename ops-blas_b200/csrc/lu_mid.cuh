@@ -17,6 +17,7 @@
 #include <cuda_runtime.h>
 
 #include "f32x2.cuh"
+#include "quotient.cuh"
 #include "small_common.cuh"
 
 namespace opsblas {
@@ -52,16 +53,6 @@ __device__ __forceinline__ float warp_absmax(float v)
     float r;
     asm volatile("redux.sync.max.abs.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
     return r;
-}
-
-// RN(1 / b) for b in [2^-60, 2^60]: one Newton step on the hardware's approximation. It equals 1.0f / b
-// for every significand and exponent of that range (compared exhaustively), without the branch that
-// the general reciprocal has.
-__device__ __forceinline__ float mid_reciprocal(float b)
-{
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
-    return fmaf(fmaf(-b, y, 1.0f), y, y);
 }
 
 // A block in registers: p[t][h] = columns 2h, 2h + 1 of row lane + 32 t, packed for the f32x2 unit
@@ -191,18 +182,12 @@ __device__ __forceinline__ void mid_apply(MidBlock<MidSmem<NBLK, W>::R>& p, MidS
 
 // Factors block jb's cw columns and publishes it: values to S, posn, rowof, ipiv. Returns the number
 // of columns eliminated (cw, or the column of the block at which the pivot is exactly zero).
-//
-// Multipliers: the correctly rounded a / b of many a for one b. With y = RN(1 / b), two residual
-// corrections q <- q + RN(a - q b) y give it (Markstein, "Computation of elementary functions on the
-// IBM RISC System/6000 processor", 1990: the first makes q faithful, the second rounds it) while
-// neither the quotient nor the residual can underflow: |b| in [2^-60, 2^60] and |a| >= 2^-60. Other
-// values (zeros among them, whose sign the corrections lose) take the division; NaN stays NaN on both.
+// Multipliers are quotients by one reciprocal (quotient.cuh).
 template <int NBLK, bool PIVOT, int W>
 __device__ __forceinline__ int mid_factor(MidBlock<MidSmem<NBLK, W>::R>& p, MidSmem<NBLK, W>& M, float* u, int n,
                                           int jb, int cw, int lane)
 {
     constexpr int R = MidSmem<NBLK, W>::R, LD = MidSmem<NBLK, W>::LD;
-    constexpr float lo = 0x1p-60f, hi = 0x1p60f;
     const int k0 = jb * kMidNB;
     int pos[R];    // the rows' positions (255: no row)
     bool live[R];  // rows of the panel: alive before it
@@ -230,8 +215,8 @@ __device__ __forceinline__ int mid_factor(MidBlock<MidSmem<NBLK, W>::R>& p, MidS
 #pragma unroll
             for (int t = 1; t < R; t++) best = fmaxf(best, fabsf(a[t]));
             const float mx = warp_absmax(best);
-            y = mid_reciprocal(mx);
-            usual = mx >= lo && mx <= hi;
+            y = qt_reciprocal(mx);
+            usual = qt_usual(mx);
             unsigned cand = 0xffffffffu;
 #pragma unroll
             for (int t = 0; t < R; t++)
@@ -260,22 +245,11 @@ __device__ __forceinline__ int mid_factor(MidBlock<MidSmem<NBLK, W>::R>& p, MidS
             break;
         }
         float l[R];
-        float least = 0.0f;
         if (PIVOT) {
-            y = copysignf(y, pv);
-            least = fabsf(a[0]);
+            qt_quotients<R>(a, pv, copysignf(y, pv), usual, l);
+        } else {
 #pragma unroll
-            for (int t = 0; t < R; t++) {
-                if (t > 0) least = fminf(least, fabsf(a[t]));
-                float v = __fmul_rn(a[t], y);
-                v = fmaf(fmaf(-v, pv, a[t]), y, v);
-                l[t] = fmaf(fmaf(-v, pv, a[t]), y, v);
-            }
-        }
-        if (!usual || least < lo) {
-#pragma unroll
-            for (int t = 0; t < R; t++)
-                if (!usual || fabsf(a[t]) < lo) l[t] = a[t] / pv;
+            for (int t = 0; t < R; t++) l[t] = a[t] / pv;
         }
 #pragma unroll
         for (int t = 0; t < R; t++) {
