@@ -290,12 +290,11 @@ __device__ __forceinline__ int lu_panel_half(f32x2 (&p)[RPT][kBpH / 2], int (&po
             break;
         }
         float l[RPT];
-        if (PIVOT) {
-            qt_quotients<RPT>(a, pv, copysignf(y, pv), usual, l);
-        } else {
-#pragma unroll
-            for (int r = 0; r < RPT; r++) l[r] = a[r] / pv;
+        if (!PIVOT) {
+            usual = qt_usual(pv);
+            y = qt_reciprocal(pv);
         }
+        qt_quotients<PIVOT, RPT>(a, pv, copysignf(y, pv), usual, l);
 #pragma unroll
         for (int r = 0; r < RPT; r++) {
             const bool hit = pos[r] == ppos;

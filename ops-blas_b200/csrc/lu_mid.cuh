@@ -245,12 +245,11 @@ __device__ __forceinline__ int mid_factor(MidBlock<MidSmem<NBLK, W>::R>& p, MidS
             break;
         }
         float l[R];
-        if (PIVOT) {
-            qt_quotients<R>(a, pv, copysignf(y, pv), usual, l);
-        } else {
-#pragma unroll
-            for (int t = 0; t < R; t++) l[t] = a[t] / pv;
+        if (!PIVOT) {
+            usual = qt_usual(pv);
+            y = qt_reciprocal(pv);
         }
+        qt_quotients<PIVOT, R>(a, pv, copysignf(y, pv), usual, l);
 #pragma unroll
         for (int t = 0; t < R; t++) {
             if (pos[t] == k) pos[t] = ppos;

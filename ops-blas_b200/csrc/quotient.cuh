@@ -49,21 +49,25 @@ __device__ __forceinline__ float qt_reciprocal(float b)
     return qt_newton(b, y);
 }
 
-// l = a / b, all a no larger than b in magnitude or NaN; y = RN(1 / b) if `usual` (qt_usual(b)), which is the
-// same for the whole warp. Small numerators, and all of them for other divisors, take the division.
-template <int R>
+// l = a / b; y = RN(1 / b) if `usual` (qt_usual(b)), which is the same for the whole warp. BOUNDED: no a is
+// larger than b in magnitude (NaN aside). Numerators out of range, and all of them for other divisors, take
+// the division.
+template <bool BOUNDED, int R>
 __device__ __forceinline__ void qt_quotients(const float (&a)[R], float b, float y, bool usual, float (&l)[R])
 {
-    float least = fabsf(a[0]);
+    float least = fabsf(a[0]), most = least;
 #pragma unroll
     for (int r = 0; r < R; r++) {
-        if (r > 0) least = fminf(least, fabsf(a[r]));
+        if (r > 0) {
+            least = fminf(least, fabsf(a[r]));
+            if (!BOUNDED) most = fmaxf(most, fabsf(a[r]));
+        }
         l[r] = qt_quotient(a[r], b, y);
     }
-    if (!usual || least < qt_low) {
+    if (!usual || least < qt_low || (!BOUNDED && most > qt_high)) {
 #pragma unroll
         for (int r = 0; r < R; r++)
-            if (!usual || fabsf(a[r]) < qt_low) l[r] = a[r] / b;
+            if (!usual || fabsf(a[r]) < qt_low || (!BOUNDED && fabsf(a[r]) > qt_high)) l[r] = a[r] / b;
     }
 }
 #endif

@@ -8,7 +8,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-def _quotients(handle, n, b, a):
+def _quotients(handle, n, b, a, pivot=True):
     """The multipliers of a (batch, n - 1) for pivots b (batch), as getrf of order n forms them."""
     import torch
 
@@ -16,7 +16,7 @@ def _quotients(handle, n, b, a):
     A[:, range(1, n), range(1, n)] = 1.0
     A[:, 0, 0] = b
     A[:, 0, 1:] = a
-    handle.getrf(A, n, n)
+    handle.getrf(A, n, n, pivot=pivot)
     return A[:, 0, 1:]
 
 
@@ -66,3 +66,21 @@ def test_other_orders(handle, n):
     a[:, 8] = -0.0
     got = _quotients(handle, n, b, a)
     assert torch.equal(got.view(torch.int32), (a / b.unsqueeze(1)).view(torch.int32))
+
+
+@pytest.mark.parametrize("n", [33, 128, 129, 300])
+def test_numerators_above_the_divisor(handle, n):
+    """Without pivoting a may be larger than b: quotients up to 2^120, numerators beyond the range, not finite."""
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(n + 1)
+    b = torch.ldexp(1.0 + torch.rand(512, device="cuda", generator=g), torch.randint(-60, 61, (512,), device="cuda", generator=g))
+    b[0], b[1], b[2], b[3] = 2.0 ** -60, 2.0 ** 60, 2.0 - 2.0 ** -23, -3.0
+    shape = (512, n - 1)
+    a = torch.ldexp(1.0 + torch.rand(shape, device="cuda", generator=g), torch.randint(-70, 71, shape, device="cuda", generator=g))
+    a[:, 0], a[:, 1], a[:, 2], a[:, 3] = 2.0 ** 60, 2.0 ** -60, 0.0, -0.0
+    a[5, 4], a[6, 5] = float("inf"), float("nan")
+    want = a / b.unsqueeze(1)
+    got = _quotients(handle, n, b, a, pivot=False)
+    same = (got.view(torch.int32) == want.view(torch.int32)) | (got.isnan() & want.isnan())
+    assert bool(same.all())
