@@ -32,19 +32,12 @@ __device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c)
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
-// Each half rounded on its own. (A product that feeds a packed sum directly is joined with it into an fma
-// all the same: negate it in between where both roundings are wanted.)
+// Each half rounded on its own. There is no packed sum here: the ptxas of CUDA 12.9 joins one with a packed
+// product that feeds it into an fma, whatever roundings the two name.
 __device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b)
 {
     f32x2 r;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
-__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b)
-{
-    f32x2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
 }  // namespace opsblas

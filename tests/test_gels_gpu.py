@@ -72,6 +72,16 @@ def test_gels_warp_path_shapes(handle, shape):
     check(handle, t, a, c, m, n, nrhs, lda, ldc, f"{t} {m}x{n}x{nrhs}")
 
 
+@pytest.mark.parametrize("m", range(1, 33))
+def test_gels_every_height(handle, m):
+    """The warp kernel is one instantiation a row count; as test_geqrf_every_height."""
+    rng = np.random.default_rng(m)
+    for n, nrhs, lda in ((min(m, 16), 3, m), (max(1, m // 2), 32 - max(1, m // 2), m + 1)):
+        a = rng.standard_normal((40, n, lda)).astype(np.float32)
+        c = rng.standard_normal((40, nrhs, lda)).astype(np.float32)
+        check(handle, "N", a, c, m, n, nrhs, lda, lda, f"{m}x{n}x{nrhs} lda {lda}")
+
+
 def test_gels_large_batch(handle):
     row = ("big", "N", 32, 16, 2, 32, 32, 4096, "RANDOM", "-", "SUCCESS", "overdetermined")
     a, c = gels_inputs(row, 5)

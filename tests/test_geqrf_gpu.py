@@ -53,6 +53,14 @@ def test_geqrf_shapes_with_padding(handle, mn):
     check(handle, a, m, n, lda, f"{m}x{n}")
 
 
+@pytest.mark.parametrize("m", range(1, 33))
+def test_geqrf_every_height(handle, m):
+    """The register kernel is one instantiation a row count, odd and even, aligned columns or not: a product and a
+    difference that a compiler joined would show in the last bits of the update."""
+    for n, lda in ((32, m), (9, m + 4 - m % 4), (17, m + 1)):
+        check(handle, geqrf_matrices(m, n, lda, "RANDOM_NORM_2", m * 64 + n, 40), m, n, lda, f"{m}x{n} lda {lda}")
+
+
 def test_geqrf_chain_scale_reconstruction(handle):
     import torch
 
