@@ -24,6 +24,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "internal.h"
@@ -70,16 +71,34 @@ __device__ __forceinline__ void grouped_mid(const GroupDev& g, int li, float* co
     team_sync<W * 32>(bar + W);
     mid_getrf<NBLK, true, W, 0>(M, n, warp, lane, bar);
     team_sync<W * 32>(bar + W);
-    for (int c = warp; c < g.nrhs; c += W) {
+    // column c + i W, i < C; those past the last one repeat it
+    auto solve = [&](auto count, int c) {
+        constexpr int C = decltype(count)::value;
+        const int last = (g.nrhs - 1 - c) / W;
         float* bc = Barray[inst] + (long long)c * g.ldb;
-        float y[R];
+        float y[C][R];
 #pragma unroll
-        for (int t = 0; t < R; t++) y[t] = lane + 32 * t < n ? bc[M.rowof[lane + 32 * t]] : 0.0f;
+        for (int t = 0; t < R; t++) {
+            const int r = lane + 32 * t < n ? M.rowof[lane + 32 * t] : -1;
+#pragma unroll
+            for (int i = 0; i < C; i++) y[i][t] = r >= 0 ? bc[r + (long long)(min(i, last) * W) * g.ldb] : 0.0f;
+        }
         __syncwarp();  // every lane has read its b before any lane writes x
-        mid_solve<NBLK, W>(M, n, lane, y);
+        mid_solve<NBLK, W, C>(M, n, lane, y);
 #pragma unroll
-        for (int t = 0; t < R; t++)
-            if (lane + 32 * t < n) bc[lane + 32 * t] = y[t];
+        for (int i = 0; i < C; i++) {
+            if (i > last) break;
+#pragma unroll
+            for (int t = 0; t < R; t++)
+                if (lane + 32 * t < n) bc[lane + 32 * t + (long long)(i * W) * g.ldb] = y[i][t];
+        }
+    };
+    if (g.nrhs > 2 * W) {
+        for (int c = warp; c < g.nrhs; c += 4 * W) solve(std::integral_constant<int, 4>{}, c);
+    } else if (g.nrhs > W) {
+        solve(std::integral_constant<int, 2>{}, warp);
+    } else if (warp < g.nrhs) {
+        solve(std::integral_constant<int, 1>{}, warp);
     }
     mid_store<NBLK, W>(M, A, g.lda, n, piv + g.piv_off + (long long)li * n, warp, lane);
     if (warp == 0 && lane == 0) info[inst] = M.stop < n ? M.stop + 1 : 0;

@@ -410,11 +410,13 @@ __device__ __forceinline__ void mid_store(const MidSmem<NBLK, W>& M, float* A, i
     }
 }
 
-// One right-hand side solved by one warp from the factors in M.S, in the reference getrs's order
-// (trans N): y[t] enters as b[rowof[lane + 32 t]] and leaves as x[lane + 32 t].
-template <int NBLK, int W>
+// C right-hand sides solved by one warp from the factors in M.S, in the reference getrs's order (trans N):
+// y[c][t] enters as b[rowof[lane + 32 t]] and leaves as x[lane + 32 t]. A step is a chain of a broadcast, an
+// fma and in the U sweep a division: four columns at a time hide it (us, orders 80, 8 columns, 100 instances
+// in one grouped launch: 158 with one at a time, 107).
+template <int NBLK, int W, int C>
 __device__ __forceinline__ void mid_solve(const MidSmem<NBLK, W>& M, int n, int lane,
-                                          float (&y)[MidSmem<NBLK, W>::R])
+                                          float (&y)[C][MidSmem<NBLK, W>::R])
 {
     constexpr int R = MidSmem<NBLK, W>::R, LD = MidSmem<NBLK, W>::LD;
     const float* s[R];
@@ -426,10 +428,16 @@ __device__ __forceinline__ void mid_solve(const MidSmem<NBLK, W>& M, int n, int 
         for (int l = 0; l < 32; l++) {
             const int k = 32 * q + l;
             if (k >= n) break;
-            const float yk = __shfl_sync(0xffffffffu, y[q], l);
-            if (lane > l) y[q] = fmaf(-s[q][k * LD], yk, y[q]);
+            float m[R];
 #pragma unroll
-            for (int t = q + 1; t < R; t++) y[t] = fmaf(-s[t][k * LD], yk, y[t]);
+            for (int t = q; t < R; t++) m[t] = -s[t][k * LD];
+#pragma unroll
+            for (int c = 0; c < C; c++) {
+                const float yk = __shfl_sync(0xffffffffu, y[c][q], l);
+                if (lane > l) y[c][q] = fmaf(m[q], yk, y[c][q]);
+#pragma unroll
+                for (int t = q + 1; t < R; t++) y[c][t] = fmaf(m[t], yk, y[c][t]);
+            }
         }
     }
 #pragma unroll
@@ -439,10 +447,16 @@ __device__ __forceinline__ void mid_solve(const MidSmem<NBLK, W>& M, int n, int 
 #pragma unroll 4
         for (int l = min(31, n - 1 - 32 * q); l >= 0; l--) {
             const int k = 32 * q + l;
-            const float xk = __shfl_sync(0xffffffffu, y[q] / diag, l);
-            y[q] = lane == l ? xk : (lane < l ? fmaf(-s[q][k * LD], xk, y[q]) : y[q]);
+            float m[R];
 #pragma unroll
-            for (int t = 0; t < q; t++) y[t] = fmaf(-s[t][k * LD], xk, y[t]);
+            for (int t = 0; t <= q; t++) m[t] = -s[t][k * LD];
+#pragma unroll
+            for (int c = 0; c < C; c++) {
+                const float xk = __shfl_sync(0xffffffffu, y[c][q] / diag, l);
+                y[c][q] = lane == l ? xk : (lane < l ? fmaf(m[q], xk, y[c][q]) : y[c][q]);
+#pragma unroll
+                for (int t = 0; t < q; t++) y[c][t] = fmaf(m[t], xk, y[c][t]);
+            }
         }
     }
 }
