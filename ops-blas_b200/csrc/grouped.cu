@@ -182,7 +182,41 @@ __device__ __forceinline__ void grouped_small_dispatch(const GroupDev& g, const 
         grouped_small<N, 32>(g, task, Aarray, Barray, piv, info, rowbuf, owner, lane);
 }
 
-// Tasks of one class, taken by the CTA's teams from the class's counter.
+// Tasks of n <= 32, a warp each: the CTA takes as many neighbours of the list as it has warps at a time, which
+// are mostly of one order. Their code is long and runs once a task, so that an SM whose warps took
+// scattered tasks waited for instructions (400 orders of 4 to 32: 46 us; together 23).
+template <int WARPS, bool FIRST>
+__device__ __forceinline__ void grouped_small_tasks(const GroupDev* groups, const GroupTask* __restrict__ tasks,
+                                                    int count, int* counter, float* const* Aarray,
+                                                    float* const* Barray, int* piv, int* info, float* rowbuf, int* owner,
+                                                    int* s_task, int wid, int lane)
+{
+    // FIRST: the CTA's first tasks are its own, and the counter deals out those after all CTAs' first
+    for (bool first = FIRST;; first = false) {
+        if (threadIdx.x == 0)
+            *s_task = first ? (int)blockIdx.x * WARPS : atomicAdd(counter, WARPS) + (FIRST ? (int)gridDim.x * WARPS : 0);
+        __syncthreads();
+        const int t0 = *s_task;
+        if (t0 >= count) break;  // uniform
+        if (t0 + wid < count) {
+            const GroupTask task = tasks[t0 + wid];
+            const GroupDev& g = groups[task.group];  // fields read when needed: fewer live registers
+            switch (g.n) {
+#define OPSBLAS_GROUPED_CASE(NN)                                                                                    \
+    case NN:                                                                                                        \
+        grouped_small_dispatch<NN>(g, task, Aarray, Barray, piv, info, rowbuf, owner, lane);                        \
+        break;
+                OPSBLAS_FOR_N_1_32(OPSBLAS_GROUPED_CASE)
+#undef OPSBLAS_GROUPED_CASE
+                default:
+                    break;
+            }
+        }
+        __syncthreads();  // the tasks' number is read, and shared memory free, before the next
+    }
+}
+
+// Tasks of one class of n > 32, taken by the CTA's teams from the class's counter.
 template <int C>
 __device__ __forceinline__ void grouped_class(const GroupDev* groups, const GroupTask* __restrict__ tasks, int count,
                                               int* counter, float* const* Aarray, float* const* Barray, int* piv,
@@ -209,24 +243,11 @@ __device__ __forceinline__ void grouped_class(const GroupDev* groups, const Grou
         const GroupDev& g = groups[task.group];  // fields read when needed: fewer live registers
         if constexpr (C < 4) {
             grouped_mid<8 - C, W>(g, task.first, Aarray, Barray, piv, info, region, warp, lane, bar);
-        } else if constexpr (C == 4) {
+        } else {
             if (g.n > 48)
                 grouped_mid<4, W>(g, task.first, Aarray, Barray, piv, info, region, warp, lane, bar);
             else
                 grouped_mid<3, W>(g, task.first, Aarray, Barray, piv, info, region, warp, lane, bar);
-        } else {
-            float* rowbuf = reinterpret_cast<float*>(region);
-            int* owner = reinterpret_cast<int*>(rowbuf + 64);
-            switch (g.n) {
-#define OPSBLAS_GROUPED_CASE(NN)                                                                                    \
-    case NN:                                                                                                        \
-        grouped_small_dispatch<NN>(g, task, Aarray, Barray, piv, info, rowbuf, owner, lane);                        \
-        break;
-                OPSBLAS_FOR_N_1_32(OPSBLAS_GROUPED_CASE)
-#undef OPSBLAS_GROUPED_CASE
-                default:
-                    break;
-            }
         }
     }
 }
@@ -237,6 +258,18 @@ __device__ __forceinline__ void grouped_class(const GroupDev* groups, const Grou
 struct GroupLists {
     int first[kGrpClasses + 1];
 };
+
+// The last CTA out resets the counters for the next execution.
+__device__ __forceinline__ void grouped_last_out(int* counters)
+{
+    if (threadIdx.x == 0) {
+        __threadfence();
+        const int f = atomicAdd(&counters[kGrpClasses], 1);
+        if (f == (int)gridDim.x - 1) {
+            for (int c = 0; c <= kGrpClasses; c++) atomicExch(&counters[c], 0);
+        }
+    }
+}
 
 __global__ void __launch_bounds__(kGrpThreads, 1)
 grouped_lu_kernel(const GroupDev* groups, const GroupTask* __restrict__ tasks, const GroupLists lists,
@@ -256,17 +289,32 @@ grouped_lu_kernel(const GroupDev* groups, const GroupTask* __restrict__ tasks, c
     OPSBLAS_GROUPED_CLASS(2)
     OPSBLAS_GROUPED_CLASS(3)
     OPSBLAS_GROUPED_CLASS(4)
-    OPSBLAS_GROUPED_CLASS(5)
 #undef OPSBLAS_GROUPED_CLASS
-
-    // the last CTA out resets the counters for the next execution
-    if (threadIdx.x == 0) {
-        __threadfence();
-        const int f = atomicAdd(&counters[kGrpClasses], 1);
-        if (f == (int)gridDim.x - 1) {
-            for (int c = 0; c <= kGrpClasses; c++) atomicExch(&counters[c], 0);
-        }
+    constexpr int S = kGrpClasses - 1;
+    if (lists.first[S + 1] > lists.first[S]) {
+        float* rowbuf = reinterpret_cast<float*>(dyn + (size_t)wid * grp_region(S));
+        grouped_small_tasks<kGrpWarps, false>(groups, tasks + lists.first[S], lists.first[S + 1] - lists.first[S],
+                                              counters + S, Aarray, Barray, piv, info, rowbuf,
+                                              reinterpret_cast<int*>(rowbuf + 64), s_task, wid, lane);
     }
+    grouped_last_out(counters);
+}
+
+// A plan of orders up to 32 only: nothing needs the shared memory or the registers of the classes above, and
+// sixteen warps an SM in two CTAs hide more latency than twelve (20000 orders: @@SMALL@@).
+constexpr int kGrpSmallWarps = 8;
+
+__global__ void __launch_bounds__(kGrpSmallWarps * 32, 2)
+grouped_small_kernel(const GroupDev* groups, const GroupTask* __restrict__ tasks, int count, int* __restrict__ counters,
+                     float* const* Aarray, float* const* Barray, int* piv, int* info)
+{
+    __shared__ __align__(16) float rowbuf[kGrpSmallWarps][64];
+    __shared__ int owner[kGrpSmallWarps][32];
+    __shared__ int s_task;
+    const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    grouped_small_tasks<kGrpSmallWarps, true>(groups, tasks, count, counters + kGrpClasses - 1, Aarray, Barray, piv,
+                                              info, rowbuf[wid], owner[wid], &s_task, wid, lane);
+    grouped_last_out(counters);
 }
 
 // ------------------------------------------------------------------------- host side --
@@ -370,6 +418,7 @@ struct _aclblas_grouped_plan {
     int grid = 0;
     size_t smem = 0;      // dynamic shared memory per CTA
     bool has_persistent = false;
+    bool small_only = false;  // every task has n <= 32
 };
 
 using namespace opsblas;
@@ -459,6 +508,7 @@ extern "C" aclblasStatus_t aclblasSgetrfGetrsGroupedPlanCreate(aclblasHandle_t h
     }
     while (cls < kGrpClasses) p->lists.first[++cls] = (int)tasks.size();
     p->has_persistent = !tasks.empty();
+    p->small_only = p->lists.first[kGrpClasses - 1] == 0;
     p->smem = smem;
 
     std::vector<GroupDev> gd(std::max(groupCount, 1));
@@ -482,18 +532,23 @@ extern "C" aclblasStatus_t aclblasSgetrfGetrsGroupedPlanCreate(aclblasHandle_t h
         err = cudaMemset(p->d_counters, 0, 256);
         if (err == cudaSuccess) err = cudaMemcpy(p->d_groups, gd.data(), bg, cudaMemcpyHostToDevice);
         if (err == cudaSuccess) err = cudaMemcpy(p->d_tasks, tasks.data(), bt, cudaMemcpyHostToDevice);
-        if (err == cudaSuccess)
-            err = ensure_smem_limit(grouped_lu_kernel, (int)std::max<size_t>(p->smem, 1));
         int per_sm = 0;
-        if (err == cudaSuccess)
-            err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grouped_lu_kernel, kGrpThreads, p->smem);
+        if (err == cudaSuccess && p->small_only) {
+            err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grouped_small_kernel, kGrpSmallWarps * 32, 0);
+        } else if (err == cudaSuccess) {
+            err = ensure_smem_limit(grouped_lu_kernel, (int)p->smem);
+            if (err == cudaSuccess)
+                err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grouped_lu_kernel, kGrpThreads, p->smem);
+        }
         if (err != cudaSuccess || per_sm < 1) {
             log_error(kApi, "plan set-up failed: %s", cudaGetErrorString(err));
             cudaFree(p->dmem);
             delete p;
             return err != cudaSuccess ? launch_status(kApi, err) : ACLBLAS_STATUS_NOT_SUPPORTED;
         }
-        p->grid = (int)std::min<long long>((long long)tasks.size(), sm_count());
+        const long long ctas = p->small_only ? ((long long)tasks.size() + kGrpSmallWarps - 1) / kGrpSmallWarps
+                                             : (long long)tasks.size();
+        p->grid = (int)std::min<long long>(ctas, (long long)(p->small_only ? per_sm : 1) * sm_count());
     }
     *plan = p;
     return ACLBLAS_STATUS_SUCCESS;
@@ -541,8 +596,13 @@ extern "C" aclblasStatus_t aclblasSgetrfGetrsGroupedBatched(aclblasHandle_t hand
     }
     cudaStream_t st = handle->stream;
     if (plan->has_persistent) {
-        grouped_lu_kernel<<<(unsigned)plan->grid, kGrpThreads, plan->smem, st>>>(
-            plan->d_groups, plan->d_tasks, plan->lists, plan->d_counters, Aarray, Barray, PivotArray, infoArray);
+        if (plan->small_only)
+            grouped_small_kernel<<<(unsigned)plan->grid, kGrpSmallWarps * 32, 0, st>>>(
+                plan->d_groups, plan->d_tasks, plan->lists.first[kGrpClasses], plan->d_counters, Aarray, Barray,
+                PivotArray, infoArray);
+        else
+            grouped_lu_kernel<<<(unsigned)plan->grid, kGrpThreads, plan->smem, st>>>(
+                plan->d_groups, plan->d_tasks, plan->lists, plan->d_counters, Aarray, Barray, PivotArray, infoArray);
         cudaError_t err = cudaGetLastError();
         if (err != cudaSuccess) return launch_status(kApi, err);
     }

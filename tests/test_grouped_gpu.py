@@ -112,6 +112,17 @@ def test_grouped_every_config_gives_the_same_bits(ob, handle, config):
                 assert (warps, rows) == (config[1], config[2])
 
 
+@pytest.mark.parametrize("sizes", [[1], [7], [8], [9], [3, 70, 41, 5, 1, 2], [900, 2, 1501, 333, 64, 3000]])
+def test_grouped_small_orders_only(ob, handle, sizes):
+    """Plans of orders up to 32 (a kernel of their own, eight tasks a CTA at a time): fewer tasks than a CTA has
+    warps, remainders, several rounds of every CTA, and twice over."""
+    ns = [32, 17, 9, 8, 4, 1][: len(sizes)]
+    d = _setup(ob, ns=ns, nrhss=[1, 3, 0, 2, 1, 1][: len(sizes)], sizes=sizes, seed=11)
+    out, ref, _ = _run_both(ob, handle, d, repeats=2)
+    for o in out:
+        _assert_same(o, ref)
+
+
 def test_grouped_singular_and_factor_only(ob, handle):
     ns = [5, 16, 32, 40, 96, 128]
     d = _setup(ob, ns=ns, nrhss=[1, 0, 2, 1, 0, 1], sizes=[6, 6, 6, 6, 6, 6], seed=4,
