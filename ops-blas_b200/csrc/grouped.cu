@@ -219,7 +219,7 @@ __device__ __forceinline__ void grouped_small_tasks(const GroupDev* groups, cons
 // Tasks of one class of n > 32, taken by the CTA's teams from the class's counter.
 template <int C>
 __device__ __forceinline__ void grouped_class(const GroupDev* groups, const GroupTask* __restrict__ tasks, int count,
-                                              int* counter, float* const* Aarray, float* const* Barray, int* piv,
+                                              bool only, int* counter, float* const* Aarray, float* const* Barray, int* piv,
                                               int* info, unsigned char* dyn, int* s_task, int wid, int lane)
 {
     constexpr int W = grp_team_warps(C);
@@ -227,14 +227,18 @@ __device__ __forceinline__ void grouped_class(const GroupDev* groups, const Grou
     if (team >= grp_teams(C)) return;
     const int bar = 1 + team * (W + 1);
     unsigned char* region = dyn + (size_t)team * grp_region(C);
-    for (;;) {
+    // only: there is no other class. Every SM's first team, then its second, and so on, take the first tasks;
+    // asked for, they go to the SMs that start first (400 orders of 33 to 64: 67 us, 54). With classes to
+    // follow that is as well: the other SMs go on to those meanwhile (400 of 65 to 96: 82 us, 125).
+    const int spread = only ? grp_teams(C) * (int)gridDim.x : 0;
+    for (bool first = only;; first = false) {
         team_sync<W * 32>(bar + W);  // the previous task's shared memory and task number are done with
-        int t;
-        if (W == 1) {
-            t = lane == 0 ? atomicAdd(counter, 1) : 0;
+        int t = team * (int)gridDim.x + (int)blockIdx.x;
+        if (!first && W == 1) {
+            t = lane == 0 ? atomicAdd(counter, 1) + spread : 0;
             t = __shfl_sync(0xffffffffu, t, 0);
-        } else {
-            if (warp == 0 && lane == 0) s_task[team] = atomicAdd(counter, 1);
+        } else if (!first) {
+            if (warp == 0 && lane == 0) s_task[team] = atomicAdd(counter, 1) + spread;
             team_sync<W * 32>(bar + W);
             t = s_task[team];
         }
@@ -280,8 +284,9 @@ grouped_lu_kernel(const GroupDev* groups, const GroupTask* __restrict__ tasks, c
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #define OPSBLAS_GROUPED_CLASS(C)                                                                                    \
     if (lists.first[C + 1] > lists.first[C]) {                                                                      \
-        grouped_class<C>(groups, tasks + lists.first[C], lists.first[C + 1] - lists.first[C], counters + C, Aarray, \
-                         Barray, piv, info, dyn, s_task, wid, lane);                                                \
+        const int count = lists.first[C + 1] - lists.first[C];                                                      \
+        grouped_class<C>(groups, tasks + lists.first[C], count, count == lists.first[kGrpClasses], counters + C,    \
+                         Aarray, Barray, piv, info, dyn, s_task, wid, lane);                                        \
         __syncthreads();                                                                                            \
     }
     OPSBLAS_GROUPED_CLASS(0)
@@ -301,7 +306,7 @@ grouped_lu_kernel(const GroupDev* groups, const GroupTask* __restrict__ tasks, c
 }
 
 // A plan of orders up to 32 only: nothing needs the shared memory or the registers of the classes above, and
-// sixteen warps an SM in two CTAs hide more latency than twelve (20000 orders: @@SMALL@@).
+// sixteen warps an SM in two CTAs hide more latency than twelve (20000 orders of 4 to 32: 123 us, 98).
 constexpr int kGrpSmallWarps = 8;
 
 __global__ void __launch_bounds__(kGrpSmallWarps * 32, 2)

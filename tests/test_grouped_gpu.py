@@ -123,6 +123,18 @@ def test_grouped_small_orders_only(ob, handle, sizes):
         _assert_same(o, ref)
 
 
+@pytest.mark.parametrize("ns,sizes", [([128], [3]), ([113, 120], [200, 300]), ([100], [700]), ([81, 96], [1, 900]),
+                                      ([70], [1200]), ([33, 48, 49, 64], [700, 600, 500, 1])])
+def test_grouped_one_class(ob, handle, ns, sizes):
+    """Orders of one class alone, whose first tasks are dealt out in advance: fewer instances than SMs, more than
+    the first tasks of all teams; one, two and eight columns (one, two and four at a time in a warp); twice."""
+    for nrhs in (1, 2, 8):
+        d = _setup(ob, ns=ns, nrhss=[nrhs] * len(ns), sizes=sizes, seed=len(ns) + nrhs)
+        out, ref, _ = _run_both(ob, handle, d, repeats=2)
+        for o in out:
+            _assert_same(o, ref)
+
+
 def test_grouped_singular_and_factor_only(ob, handle):
     ns = [5, 16, 32, 40, 96, 128]
     d = _setup(ob, ns=ns, nrhss=[1, 0, 2, 1, 0, 1], sizes=[6, 6, 6, 6, 6, 6], seed=4,
