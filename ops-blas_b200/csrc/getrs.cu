@@ -27,10 +27,11 @@ namespace opsblas {
 // thread per right-hand side (the reference's order); the other sweeps run in parallel over
 // (row, rhs) with one barrier per pivot step.
 constexpr int kGenericThreads = 256;
+constexpr int kGenericRhs = 256;  // right-hand sides a pass (plans and refinements may have more)
 
 __global__ void __launch_bounds__(kGenericThreads)
 getrs_generic_kernel(const float* const* __restrict__ Aarray, int n, int lda, const int* __restrict__ ipiv,
-                     float* const* __restrict__ Barray, int ldb, int nrhs, int trans)
+                     float* const* __restrict__ Barray, int ldb, int allrhs, int trans)
 {
     const long long m = blockIdx.x;
     const float* A = Aarray[m];
@@ -38,84 +39,88 @@ getrs_generic_kernel(const float* const* __restrict__ Aarray, int n, int lda, co
     if (B == nullptr) return;  // a NULL right-hand side skips the matrix
     const int* p = ipiv ? ipiv + m * n : nullptr;
     const int tid = threadIdx.x;
-    __shared__ float sx[256];
-    auto at = [&](int i, int j) { return A[i + (long long)j * lda]; };
-    auto bb = [&](int i, int c) -> float& { return B[i + (long long)c * ldb]; };
+    __shared__ float sx[kGenericRhs];
+    for (int c0 = 0; c0 < allrhs; c0 += kGenericRhs, B += (long long)kGenericRhs * ldb) {
+        const int nrhs = min(kGenericRhs, allrhs - c0);
+        auto at = [&](int i, int j) { return A[i + (long long)j * lda]; };
+        auto bb = [&](int i, int c) -> float& { return B[i + (long long)c * ldb]; };
 
-    auto swap_rows = [&](bool reverse) {
-        if (!p) return;
-        for (int c = tid; c < nrhs; c += kGenericThreads) {
-            for (int t = 0; t < n; t++) {
-                const int k = reverse ? n - 1 - t : t;
-                const int pk = p[k] - 1;
-                if (pk >= 0 && pk < n && pk != k) {
-                    const float tmp = bb(k, c);
-                    bb(k, c) = bb(pk, c);
-                    bb(pk, c) = tmp;
+        auto swap_rows = [&](bool reverse) {
+            if (!p) return;
+            for (int c = tid; c < nrhs; c += kGenericThreads) {
+                for (int t = 0; t < n; t++) {
+                    const int k = reverse ? n - 1 - t : t;
+                    const int pk = p[k] - 1;
+                    if (pk >= 0 && pk < n && pk != k) {
+                        const float tmp = bb(k, c);
+                        bb(k, c) = bb(pk, c);
+                        bb(pk, c) = tmp;
+                    }
                 }
             }
-        }
-    };
+        };
 
-    if (trans == 0) {
-        swap_rows(false);
-        __syncthreads();
-        for (int j = 0; j < n - 1; j++) {
-            const int rows = n - 1 - j;
-            const int total = rows * nrhs;
-            const float* lj = A + (long long)j * lda;
-            for (int idx = tid; idx < total; idx += kGenericThreads) {
-                const int c = idx / rows;
-                const int i = j + 1 + idx % rows;
-                bb(i, c) = fmaf(-lj[i], bb(j, c), bb(i, c));
-            }
+        if (trans == 0) {
+            swap_rows(false);
             __syncthreads();
-        }
-        for (int j = n - 1; j >= 0; j--) {
-            const float ujj = at(j, j);
-            for (int c = tid; c < nrhs; c += kGenericThreads) {
-                const float v = bb(j, c) / ujj;
-                bb(j, c) = v;
-                sx[c] = v;
-            }
-            __syncthreads();
-            const int total = j * nrhs;
-            const float* uj = A + (long long)j * lda;
-            for (int idx = tid; idx < total; idx += kGenericThreads) {
-                const int c = idx / j;
-                const int i = idx % j;
-                bb(i, c) = fmaf(-uj[i], sx[c], bb(i, c));
-            }
-            __syncthreads();
-        }
-    } else {
-        for (int j = 0; j < n; j++) {
-            const float ujj = at(j, j);
-            for (int c = tid; c < nrhs; c += kGenericThreads) {
-                const float v = bb(j, c) / ujj;
-                bb(j, c) = v;
-                sx[c] = v;
-            }
-            __syncthreads();
-            const int rows = n - 1 - j;
-            const int total = rows * nrhs;
-            for (int idx = tid; idx < total; idx += kGenericThreads) {
-                const int c = idx / rows;
-                const int i = j + 1 + idx % rows;
-                bb(i, c) = fmaf(-at(j, i), sx[c], bb(i, c));
-            }
-            __syncthreads();
-        }
-        for (int c = tid; c < nrhs; c += kGenericThreads) {
-            for (int j = n - 1; j >= 0; j--) {
-                float s = bb(j, c);
+            for (int j = 0; j < n - 1; j++) {
+                const int rows = n - 1 - j;
+                const int total = rows * nrhs;
                 const float* lj = A + (long long)j * lda;
-                for (int i = j + 1; i < n; i++) s = fmaf(-lj[i], bb(i, c), s);
-                bb(j, c) = s;
+                for (int idx = tid; idx < total; idx += kGenericThreads) {
+                    const int c = idx / rows;
+                    const int i = j + 1 + idx % rows;
+                    bb(i, c) = fmaf(-lj[i], bb(j, c), bb(i, c));
+                }
+                __syncthreads();
             }
+            for (int j = n - 1; j >= 0; j--) {
+                const float ujj = at(j, j);
+                for (int c = tid; c < nrhs; c += kGenericThreads) {
+                    const float v = bb(j, c) / ujj;
+                    bb(j, c) = v;
+                    sx[c] = v;
+                }
+                __syncthreads();
+                const int total = j * nrhs;
+                const float* uj = A + (long long)j * lda;
+                for (int idx = tid; idx < total; idx += kGenericThreads) {
+                    const int c = idx / j;
+                    const int i = idx % j;
+                    bb(i, c) = fmaf(-uj[i], sx[c], bb(i, c));
+                }
+                __syncthreads();
+            }
+        } else {
+            for (int j = 0; j < n; j++) {
+                const float ujj = at(j, j);
+                for (int c = tid; c < nrhs; c += kGenericThreads) {
+                    const float v = bb(j, c) / ujj;
+                    bb(j, c) = v;
+                    sx[c] = v;
+                }
+                __syncthreads();
+                const int rows = n - 1 - j;
+                const int total = rows * nrhs;
+                for (int idx = tid; idx < total; idx += kGenericThreads) {
+                    const int c = idx / rows;
+                    const int i = j + 1 + idx % rows;
+                    bb(i, c) = fmaf(-at(j, i), sx[c], bb(i, c));
+                }
+                __syncthreads();
+            }
+            for (int c = tid; c < nrhs; c += kGenericThreads) {
+                for (int j = n - 1; j >= 0; j--) {
+                    float s = bb(j, c);
+                    const float* lj = A + (long long)j * lda;
+                    for (int i = j + 1; i < n; i++) s = fmaf(-lj[i], bb(i, c), s);
+                    bb(j, c) = s;
+                }
+            }
+            __syncthreads();
+            swap_rows(true);
         }
-        __syncthreads();
-        swap_rows(true);
+        __syncthreads();  // the pass's last sweep is done before the next one writes sx
     }
 }
 

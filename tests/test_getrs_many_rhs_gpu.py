@@ -1,7 +1,7 @@
-"""aclblasSgetrsBatched, trans N, 32 < n <= 128 with at least 65536 right-hand sides in the batch:
-one thread per right-hand side walking LU columns. Bit for bit against the oracle, for a packed
-16-byte-aligned layout and a padded odd leading dimension (the per-element load path), with some
-matrices skipped through a NULL right-hand-side pointer."""
+"""Solves with many right-hand sides. aclblasSgetrsBatched, trans N, 32 < n <= 128 with at least 65536 of them in
+the batch: bit for bit against the oracle, for a packed 16-byte-aligned layout and a padded odd leading
+dimension, with some matrices skipped through a NULL right-hand-side pointer. Refinements and plans with more
+columns than one grid, or one pass of the generic solve, takes."""
 from __future__ import annotations
 
 import numpy as np
@@ -79,3 +79,28 @@ def test_grouped_more_columns_than_one_grid_takes(ob, handle):
     with_plan.close()
     assert int(info[0]) == 0
     assert torch.equal(B.reshape(nrhs // k, k, n), few.expand(nrhs // k, k, n))
+
+
+def test_grouped_more_columns_than_a_generic_pass(ob, handle):
+    """Orders whose right-hand sides no longer fit shared memory: the generic solve's 256 columns a pass. A plan takes
+    any number of them (aclblasSgetrsBatched at most 256)."""
+    import torch
+
+    n, nrhs = 2720, 300
+    g = torch.Generator(device="cuda").manual_seed(3)
+    A = torch.randn(1, n, n, device="cuda", generator=g) + 100 * torch.eye(n, device="cuda")
+    B = torch.randn(1, nrhs, n, device="cuda", generator=g)
+    LU = A.clone()
+    piv, _ = handle.getrf(LU, n, n)
+    want = []
+    for part in (B[:, :200].clone(), B[:, 200:].clone()):
+        handle.getrs("N", LU, n, n, piv, part, part.shape[1], n)
+        want.append(part)
+    piv = torch.empty(n, dtype=torch.int32, device="cuda")
+    info = torch.empty(1, dtype=torch.int32, device="cuda")
+    plan = ob.GroupedPlan(handle, [n], [nrhs], [1])
+    plan.run(handle, ob.ptr_array(A), piv, info, ob.ptr_array(B))
+    torch.cuda.synchronize()
+    plan.close()
+    assert int(info[0]) == 0
+    assert torch.equal(B, torch.cat(want, 1))
