@@ -1,18 +1,19 @@
 // aclblasSgetrfGetrsGrouped*: factor and solve many matrices of different orders in one
 // persistent launch. No counterpart in the reference (an extension beside the drop-in chain);
 // per instance the results are bit-identical to aclblasSgetrfBatched followed by
-// aclblasSgetrsBatched (trans N) on the same matrix, because the same LU and solve building
-// blocks (lu_core.cuh) run here.
+// aclblasSgetrsBatched (trans N) on the same matrix: every element takes the same operations in the
+// same order (the factorisations are the batched kernels' own code, the solves are not).
 //
 // A plan describes the batch: groups of instances that share n, nrhs, lda and ldb. Creating it
-// chooses, per group, the lanes per matrix (n <= 32) or the warps per matrix and rows per lane
-// (32 < n <= 128) from a tuning table written by autotune_grouped.py (or from the caller),
-// orders the work largest first, and uploads the task lists to the device. Each execution is
-// then one launch of grouped_lu_kernel on the handle's stream (plus the regular batched kernels
-// for groups with n > 128): one CTA of twelve warps an SM, whose teams take tasks from a device
-// counter per class of orders, largest class first --
-//   n > 32: teams of 4, 2 or 1 warps factor one matrix in their share of the CTA's shared memory
-//     (lu_mid.cuh), solve the right-hand sides from there (mid_solve) and store LU, pivots and info;
+// chooses, per group with n <= 32, the lanes per matrix from a tuning table written by
+// autotune_grouped.py (or from the caller), orders the work largest first, and uploads the task lists
+// to the device. Each execution is then one launch on the handle's stream (plus the regular batched
+// kernels for groups with n > 128). Orders up to 32 alone: grouped_small_kernel (which also follows as a
+// second launch when a mixed plan has many of them). Otherwise grouped_lu_kernel, one CTA of twelve warps an SM, whose teams take tasks from a device counter per
+// class of orders, largest class first --
+//   n > 32: teams of 4, 2 or 1 warps (by the class) factor one matrix in their share of the CTA's
+//     shared memory (lu_mid.cuh), solve the right-hand sides from there (mid_solve) and store LU,
+//     pivots and info;
 //   n <= 32: each warp takes 32/lanes matrices, factors them in registers (small_getrf_core) and
 //     solves from the registers (small_solve_core).
 // The last CTA to finish resets the counters, so consecutive executions on one stream need no
@@ -182,37 +183,38 @@ __device__ __forceinline__ void grouped_small_dispatch(const GroupDev& g, const 
         grouped_small<N, 32>(g, task, Aarray, Barray, piv, info, rowbuf, owner, lane);
 }
 
-// Tasks of n <= 32, a warp each: the CTA takes as many neighbours of the list as it has warps at a time, which
-// are mostly of one order. Their code is long and runs once a task, so that an SM whose warps took
-// scattered tasks waited for instructions (400 orders of 4 to 32: 46 us; together 23).
+// Tasks of n <= 32, a warp each. A CTA's warps start with neighbours of the list, which are mostly of one
+// order: the code of an order is long and runs once a task, so that an SM whose warps took scattered tasks
+// waited for instructions (400 orders of 4 to 32: 46 us; together 20). After that each warp asks for itself.
+// FIRST: the CTAs start together, and their first tasks need no counter.
 template <int WARPS, bool FIRST>
 __device__ __forceinline__ void grouped_small_tasks(const GroupDev* groups, const GroupTask* __restrict__ tasks,
                                                     int count, int* counter, float* const* Aarray,
                                                     float* const* Barray, int* piv, int* info, float* rowbuf, int* owner,
                                                     int* s_task, int wid, int lane)
 {
-    // FIRST: the CTA's first tasks are its own, and the counter deals out those after all CTAs' first
-    for (bool first = FIRST;; first = false) {
-        if (threadIdx.x == 0)
-            *s_task = first ? (int)blockIdx.x * WARPS : atomicAdd(counter, WARPS) + (FIRST ? (int)gridDim.x * WARPS : 0);
+    int t = (int)blockIdx.x * WARPS + wid;
+    if (!FIRST) {
+        if (threadIdx.x == 0) *s_task = atomicAdd(counter, WARPS);
         __syncthreads();
-        const int t0 = *s_task;
-        if (t0 >= count) break;  // uniform
-        if (t0 + wid < count) {
-            const GroupTask task = tasks[t0 + wid];
-            const GroupDev& g = groups[task.group];  // fields read when needed: fewer live registers
-            switch (g.n) {
+        t = *s_task + wid;
+    }
+    while (t < count) {
+        const GroupTask task = tasks[t];
+        const GroupDev& g = groups[task.group];  // fields read when needed: fewer live registers
+        switch (g.n) {
 #define OPSBLAS_GROUPED_CASE(NN)                                                                                    \
     case NN:                                                                                                        \
         grouped_small_dispatch<NN>(g, task, Aarray, Barray, piv, info, rowbuf, owner, lane);                        \
         break;
-                OPSBLAS_FOR_N_1_32(OPSBLAS_GROUPED_CASE)
+            OPSBLAS_FOR_N_1_32(OPSBLAS_GROUPED_CASE)
 #undef OPSBLAS_GROUPED_CASE
-                default:
-                    break;
-            }
+            default:
+                break;
         }
-        __syncthreads();  // the tasks' number is read, and shared memory free, before the next
+        __syncwarp();  // the warp's shared memory is read before its next task writes it
+        t = lane == 0 ? atomicAdd(counter, 1) + (FIRST ? (int)gridDim.x * WARPS : 0) : 0;
+        t = __shfl_sync(0xffffffffu, t, 0);
     }
 }
 
@@ -266,6 +268,7 @@ struct GroupLists {
 // The last CTA out resets the counters for the next execution.
 __device__ __forceinline__ void grouped_last_out(int* counters)
 {
+    __syncthreads();  // none of the CTA's warps asks for a task any more
     if (threadIdx.x == 0) {
         __threadfence();
         const int f = atomicAdd(&counters[kGrpClasses], 1);
@@ -315,10 +318,9 @@ grouped_small_kernel(const GroupDev* groups, const GroupTask* __restrict__ tasks
 {
     __shared__ __align__(16) float rowbuf[kGrpSmallWarps][64];
     __shared__ int owner[kGrpSmallWarps][32];
-    __shared__ int s_task;
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     grouped_small_tasks<kGrpSmallWarps, true>(groups, tasks, count, counters + kGrpClasses - 1, Aarray, Barray, piv,
-                                              info, rowbuf[wid], owner[wid], &s_task, wid, lane);
+                                              info, rowbuf[wid], owner[wid], nullptr, wid, lane);
     grouped_last_out(counters);
 }
 
@@ -327,8 +329,8 @@ struct TuneRow {
     int lo, hi, lanes, warps, rows;
 };
 
-// Choices for n > 32 (rows per lane, warps per matrix) that a configuration or the table may name:
-// checked and reported as ever; the kernel deals out its warps by the order alone (grp_class).
+// Rows per lane and warps per matrix for n > 32, which callers and tables may name: they have no effect (the
+// kernel deals out its warps by the order, grp_class) and are checked and reported for those that name them.
 static bool reg_shape_valid(int n, int rows, int warps)
 {
     if (n <= 32 || n > 32 * rows) return false;
@@ -423,7 +425,8 @@ struct _aclblas_grouped_plan {
     int grid = 0;
     size_t smem = 0;      // dynamic shared memory per CTA
     bool has_persistent = false;
-    bool small_only = false;  // every task has n <= 32
+    bool small_apart = false;  // the tasks of n <= 32 run in grouped_small_kernel, after the others if there are any
+    int small_grid = 0, small_first = 0, small_count = 0;  // its CTAs and tasks; grid: grouped_lu_kernel's CTAs
 };
 
 using namespace opsblas;
@@ -513,7 +516,11 @@ extern "C" aclblasStatus_t aclblasSgetrfGetrsGroupedPlanCreate(aclblasHandle_t h
     }
     while (cls < kGrpClasses) p->lists.first[++cls] = (int)tasks.size();
     p->has_persistent = !tasks.empty();
-    p->small_only = p->lists.first[kGrpClasses - 1] == 0;
+    // many small tasks repay a launch of their own, which runs sixteen warps an SM in place of twelve; fewer
+    // fill the SMs that have finished their larger orders (us, together and apart: orders of 4 to 40 with 8
+    // columns, 20000 384 and 349, 100000 1610 and 1476; of 1 to 33, 300000 1456 and 1125)
+    const int mids = p->lists.first[kGrpClasses - 1], smalls = (int)tasks.size() - mids;
+    p->small_apart = smalls > 0 && (mids == 0 || smalls >= 4 * 2 * kGrpSmallWarps * sm_count());
     p->smem = smem;
 
     std::vector<GroupDev> gd(std::max(groupCount, 1));
@@ -537,23 +544,29 @@ extern "C" aclblasStatus_t aclblasSgetrfGetrsGroupedPlanCreate(aclblasHandle_t h
         err = cudaMemset(p->d_counters, 0, 256);
         if (err == cudaSuccess) err = cudaMemcpy(p->d_groups, gd.data(), bg, cudaMemcpyHostToDevice);
         if (err == cudaSuccess) err = cudaMemcpy(p->d_tasks, tasks.data(), bt, cudaMemcpyHostToDevice);
-        int per_sm = 0;
-        if (err == cudaSuccess && p->small_only) {
-            err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grouped_small_kernel, kGrpSmallWarps * 32, 0);
-        } else if (err == cudaSuccess) {
+        int per_sm = 1, small_per_sm = 1;
+        if (err == cudaSuccess && p->small_apart)
+            err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&small_per_sm, grouped_small_kernel, kGrpSmallWarps * 32, 0);
+        if (err == cudaSuccess && !(p->small_apart && mids == 0)) {
             err = ensure_smem_limit(grouped_lu_kernel, (int)p->smem);
             if (err == cudaSuccess)
                 err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grouped_lu_kernel, kGrpThreads, p->smem);
         }
-        if (err != cudaSuccess || per_sm < 1) {
+        if (err != cudaSuccess || per_sm < 1 || small_per_sm < 1) {
             log_error(kApi, "plan set-up failed: %s", cudaGetErrorString(err));
             cudaFree(p->dmem);
             delete p;
             return err != cudaSuccess ? launch_status(kApi, err) : ACLBLAS_STATUS_NOT_SUPPORTED;
         }
-        const long long ctas = p->small_only ? ((long long)tasks.size() + kGrpSmallWarps - 1) / kGrpSmallWarps
-                                             : (long long)tasks.size();
-        p->grid = (int)std::min<long long>(ctas, (long long)(p->small_only ? per_sm : 1) * sm_count());
+        const long long lu_tasks = p->small_apart ? mids : (long long)tasks.size();
+        p->grid = (int)std::min<long long>(lu_tasks, sm_count());
+        if (p->small_apart) {
+            p->small_first = mids;
+            p->small_count = smalls;
+            p->small_grid = (int)std::min<long long>(((long long)smalls + kGrpSmallWarps - 1) / kGrpSmallWarps,
+                                                     (long long)small_per_sm * sm_count());
+            p->lists.first[kGrpClasses] = mids;  // grouped_lu_kernel leaves them alone
+        }
     }
     *plan = p;
     return ACLBLAS_STATUS_SUCCESS;
@@ -601,13 +614,13 @@ extern "C" aclblasStatus_t aclblasSgetrfGetrsGroupedBatched(aclblasHandle_t hand
     }
     cudaStream_t st = handle->stream;
     if (plan->has_persistent) {
-        if (plan->small_only)
-            grouped_small_kernel<<<(unsigned)plan->grid, kGrpSmallWarps * 32, 0, st>>>(
-                plan->d_groups, plan->d_tasks, plan->lists.first[kGrpClasses], plan->d_counters, Aarray, Barray,
-                PivotArray, infoArray);
-        else
+        if (plan->grid > 0)
             grouped_lu_kernel<<<(unsigned)plan->grid, kGrpThreads, plan->smem, st>>>(
                 plan->d_groups, plan->d_tasks, plan->lists, plan->d_counters, Aarray, Barray, PivotArray, infoArray);
+        if (plan->small_grid > 0)
+            grouped_small_kernel<<<(unsigned)plan->small_grid, kGrpSmallWarps * 32, 0, st>>>(
+                plan->d_groups, plan->d_tasks + plan->small_first, plan->small_count, plan->d_counters, Aarray, Barray,
+                PivotArray, infoArray);
         cudaError_t err = cudaGetLastError();
         if (err != cudaSuccess) return launch_status(kApi, err);
     }
