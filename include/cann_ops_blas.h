@@ -266,9 +266,9 @@ ACLBLAS_EXPORT aclblasStatus_t aclblasSgetrsAdjointBatched(
  * A plan describes groupCount groups (host arrays): group g has groupSizeArray[g] instances of
  * order nArray[g], nrhsArray[g] right-hand sides (0: factor only), leading dimensions
  * ldaArray[g] / ldbArray[g]. Instances are numbered group by group. configArray is NULL or holds
- * 3 ints per group {lanes per matrix (n <= 32: 4/8/16/32), warps per matrix (n > 32: 2, 4 or 8),
- * rows per lane (n > 32: 2, 3 or 4, with 32 * rows >= n; 2 warps only with 2 rows, 4 rows need
- * 8 warps; checked and reported as before, but the kernel deals out its warps by the order alone)},
+ * 3 ints per group {lanes per matrix (n <= 32: 4/8/16/32), warps per matrix and rows per lane
+ * (n > 32: accepted, checked and reported, without effect: the launch deals out its warps by the
+ * order; 2, 4 or 8 warps, 2, 3 or 4 rows, 32 * rows >= n, 2 warps with 2 rows, 4 rows with 8 warps)},
  * 0 = take the tuning table's choice; the table is the file
  * named by OPSBLAS_GROUPED_TUNING, else grouped_tuning.txt beside the library, else built-in
  * defaults. Invalid choices are replaced; aclblasSgetrfGetrsGroupedPlanGetConfig returns the
@@ -287,7 +287,8 @@ ACLBLAS_EXPORT aclblasStatus_t aclblasSgetrfGetrsGroupedPlanDestroy(aclblasGroup
  * (P*A = L*U, pivots at PivotArray + sum of the orders of the instances before i, infoArray[i]
  * as aclblasSgetrfBatched) and Barray[i] (n x nrhs) is overwritten by the solution X of A X = B
  * (as aclblasSgetrsBatched with trans N); the results equal those two calls bit for bit.
- * Instances with n <= 128 run in one persistent launch; larger ones use the batched kernels.
+ * Instances with n <= 128 run in one persistent launch (many of n <= 32 beside larger ones in a second);
+ * larger ones use the batched kernels.
  * No allocation and no host synchronisation. Executions of one plan must not overlap in time
  * (they share the plan's work counters). */
 ACLBLAS_EXPORT aclblasStatus_t aclblasSgetrfGetrsGroupedBatched(

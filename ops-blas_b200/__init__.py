@@ -336,8 +336,9 @@ class GroupedPlan:
     """aclblasGroupedPlan_t for groups of instances sharing (n, nrhs, lda, ldb).
 
     ``ns``, ``nrhss``, ``sizes`` (and optionally ``ldas``, ``ldbs``, default n) are per group;
-    ``config`` is None or one (lanes, warps, panel) triple per group, 0 = the tuning table's
-    choice. Instances are numbered group by group."""
+    ``config`` is None or one (lanes, warps, rows) triple per group, 0 = the tuning table's choice:
+    lanes per matrix of orders up to 32; warps and rows, for larger orders, are accepted without
+    effect. Instances are numbered group by group."""
 
     def __init__(self, handle, ns, nrhss, sizes, ldas=None, ldbs=None, config=None):
         self.ns = [int(v) for v in ns]

