@@ -13,9 +13,10 @@
 //           zeroed, Q^T applied in reverse reflector order.
 // info is per matrix (device array), as the reference kernel writes it (its CPU golden keeps one
 // value for the batch). Small QR-path systems run a warp per system (gels_warp_kernel), larger ones
-// that fit shared memory a CTA each (gels_smem_kernel); the rest one CTA per matrix in global memory: thread 0 forms each reflector, threads take the independent columns / rows /
-// right-hand sides of every step. Every sum runs in index order with each product rounded before
-// it is added -- bit for bit the CPU oracle's restatement, on both paths.
+// that fit shared memory a CTA each (gels_smem_kernel); the rest one CTA per matrix in global memory:
+// thread 0 forms each reflector, threads take the independent columns / rows / right-hand sides of
+// every step. Every sum runs in index order with each product rounded before it is added -- bit for
+// bit the CPU oracle's restatement, on all three paths.
 // Parity with the reference is its tests' rule (MERE_MARE on the solution against LAPACK sgels_).
 #include <cuda_runtime.h>
 

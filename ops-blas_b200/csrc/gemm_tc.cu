@@ -1165,8 +1165,9 @@ static cudaError_t tc_launch_t(cudaStream_t st, bool transA, bool transB, int m,
     int epi_mode = beta == 0.0f ? 1 : 2;
     if (epi_mode != 0 && !(slots && tmap_encode_c<TC>(&mc, tmslots, m, n, ldc))) epi_mode = 0;
     // One contiguous range of tiles a CTA where operands and C go by TMA and a matrix has several tiles: its
-    // maps are then set up once for them (us, every gridDim.x-th tile and this: BF16 256^3 x 1000 107 and 92,
-    // with beta 0.5 135 and 123; TF32 T N 256 x 256 x 32 x 1000 147 and 123). With a tile a matrix, or without
+    // maps are then set up once for them (us, the same operands again and again, every gridDim.x-th tile and
+    // this: BF16 256^3 x 1000 107 and 92, with beta 0.5 135 and 123; TF32 T N 256 x 256 x 32 x 1000 147 and
+    // 123. On new operands, together with the six stages: BF16 256^3 x 2048 207 and 191). With a tile a matrix, or without
     // maps to keep, the interleaved order balances better (TF32 T N 64^3 x 4000: 182, 186; FP16
     // 201 x 121 x 89 x 1024: 258, 275).
     const int contig = LU || (use_tma && epi_mode != 0 && tm * tn > 1) ? 1 : 0;

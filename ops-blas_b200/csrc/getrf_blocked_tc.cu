@@ -9,16 +9,16 @@
 //     tensor cores in split TF32.
 // Both work on the matrix stored by rows (T(i, j) at LU[j + i * ldlu]): a row is contiguous, so
 // pivot rows, interchanges and the panel's rows are whole cache lines, where by columns every row
-// element is a separate sector. The steps below describe the mixed variant; the plain one differs
-// where lu_panel_kernel's EXACT says and runs lu_rows_update_kernel as its update.
+// element is a separate sector. The steps below describe the mixed variant. The plain one has the same
+// panel, except that a stop keeps the reference's semantics and no TF32 planes are written
+// (lu_panel_kernel's EXACT), and runs lu_rows_update_kernel as its update.
 //   0. lu_rows_in_kernel: A (by columns) into LU by rows, 32 x 32 tiles through shared memory.
 //   Per panel k0 = 0, 32, ...:
 //   1. lu_panel_kernel, one CTA per matrix, two panel rows a thread:
-//      * factors the panel (rows k0..n-1, columns k0..k0+31) in FP32 in registers with implicit
-//        pivoting (`pos` tracks the reference's in-place order): pivot = the largest magnitude
-//        compared on the exponent and 14 mantissa bits (ties to the lowest position), multipliers
-//        by an approximate reciprocal -- the refinement absorbs both --, one CTA barrier per
-//        column; 1-based pivots in LAPACK's sequential-swap convention;
+//      * factors the panel (rows k0..n-1, columns k0..k0+31) in FP32 in registers, in two halves of
+//        16 columns, with implicit pivoting (`pos` tracks the reference's in-place order): the
+//        reference's first maximum of the exact magnitudes, correctly rounded multipliers, one CTA
+//        barrier per column; 1-based pivots in LAPACK's sequential-swap convention;
 //      * writes the factored panel at the final positions and moves the rest of every row whose
 //        position changed (at most 64 rows: the whole-row interchanges of the reference,
 //        SwapRows, applied once per panel);
@@ -190,8 +190,8 @@ lu_rows_out_kernel(float* const* __restrict__ LUarr, int ld, int n)
     tp_store(ta, S, ld, b0, a0, n, vec);                // S'(b0 + r, a0 + c) = ta[r][c] = S(a0 + c, b0 + r)
 }
 
-// Rows moved a round by the panel kernel's interchange step: 64 rows x MVC columns (128, or 64
-// for the small CTAs, so that their shared memory lets more of them share an SM).
+// Rows moved a round by the panel kernel's interchange step: 64 rows x MVC columns (64 for CTAs of 128 and
+// 256 threads, else 32, so that shared memory lets 512 threads of them share an SM).
 template <int NT>
 struct PanelMv {
     static constexpr int MVC = NT == 128 || NT == 256 ? 64 : 32;  // two buffers of 64 x MVC floats

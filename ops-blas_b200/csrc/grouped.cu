@@ -9,8 +9,8 @@
 // autotune_grouped.py (or from the caller), orders the work largest first, and uploads the task lists
 // to the device. Each execution is then one launch on the handle's stream (plus the regular batched
 // kernels for groups with n > 128). Orders up to 32 alone: grouped_small_kernel (which also follows as a
-// second launch when a mixed plan has many of them). Otherwise grouped_lu_kernel, one CTA of twelve warps an SM, whose teams take tasks from a device counter per
-// class of orders, largest class first --
+// second launch when a mixed plan has many of them). Otherwise grouped_lu_kernel, one CTA of twelve
+// warps an SM, whose teams take tasks from a device counter per class of orders, largest class first --
 //   n > 32: teams of 4, 2 or 1 warps (by the class) factor one matrix in their share of the CTA's
 //     shared memory (lu_mid.cuh), solve the right-hand sides from there (mid_solve) and store LU,
 //     pivots and info;

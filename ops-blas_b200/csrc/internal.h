@@ -79,7 +79,8 @@ cudaError_t getrs_launch(cudaStream_t st, bool trans, int n, int nrhs, const flo
 bool getrs_block_preferred(int n, int nrhs, int batch);
 cudaError_t getrs_block_launch(cudaStream_t st, int n, int nrhs, const float* const* Aarray, int lda, const int* ipiv,
                                float* const* Barray, int ldb, int batch);
-// getrs_blk.cu: trans N, n > 128 and some of n = 96, 128, blocked substitution with the right-hand sides in shared memory.
+// getrs_blk.cu: trans N, n > 128 and some of n = 96, 128, blocked substitution with the right-hand sides in
+// shared memory.
 bool getrs_blk_supported(int n);
 bool getrs_blk_preferred(int n, int nrhs, int batch);
 cudaError_t getrs_blk_launch(cudaStream_t st, int n, int nrhs, const float* const* Aarray, int lda, const int* ipiv,
