@@ -141,6 +141,15 @@ def test_grouped_one_class(ob, handle, ns, sizes):
             _assert_same(o, ref)
 
 
+def test_grouped_many_small_orders_beside_larger_ones(ob, handle):
+    """More small tasks than a mixed plan keeps in its one launch, beside orders of two classes; three times."""
+    ns, sizes = [100, 64, 32, 20, 3], [40, 30, 6000, 5500, 100]
+    d = _setup(ob, ns=ns, nrhss=[1, 2, 1, 1, 2], sizes=sizes, seed=12)
+    out, ref, _ = _run_both(ob, handle, d, repeats=3)
+    for o in out:
+        _assert_same(o, ref)
+
+
 def test_grouped_singular_and_factor_only(ob, handle):
     ns = [5, 16, 32, 40, 96, 128]
     d = _setup(ob, ns=ns, nrhss=[1, 0, 2, 1, 0, 1], sizes=[6, 6, 6, 6, 6, 6], seed=4,
