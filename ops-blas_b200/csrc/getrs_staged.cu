@@ -296,12 +296,11 @@ getrs_staged_kernel(const float* const* __restrict__ Aarray, int n, int lda, con
     const long long m0 = (long long)blockIdx.x * per;
     const int c0 = first + (int)blockIdx.y * cols, cw = min(cols, nrhs - c0);
 
-    bool any = false;
-    for (int g = 0; g < per; g++) any |= m0 + g < batch && Barray[m0 + g] != nullptr;
-    if (!any) return;  // nothing to solve (a refinement's converged matrices), for the whole CTA
     // LU of the CTA's matrices on its way; those without a right-hand side (NULL) are skipped
+    bool any = false;
     for (int g = 0; g < per; g++) {
         if (m0 + g >= batch || Barray[m0 + g] == nullptr) continue;
+        any = true;
         const float* A = Aarray[m0 + g];
         float* s = sm + g * region;
         if ((lda & 3) == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0) {
@@ -331,6 +330,7 @@ getrs_staged_kernel(const float* const* __restrict__ Aarray, int n, int lda, con
                     s[n + lane + j * n8] = 0.0f;
         }
     }
+    if (!any) return;  // nothing to solve (a refinement's converged matrices), for the whole CTA
     // B behind it; pivots of rows past n and invalid ones swap nothing
     for (int v = warp; v < per * cw; v += WARPS) {
         const int g = v / cw, c = v - g * cw;
